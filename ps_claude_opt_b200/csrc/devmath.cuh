@@ -10,14 +10,21 @@ namespace psb {
 // correct bits.  The facet terms only ever see d = mu + mu0 in (2e-8, 2] or
 // the stand-in 1.  Agrees with the correctly rounded 1.0 / d to within one
 // unit in the last place (checked by the test suite).
-__device__ __forceinline__ double rcp_nr(double d)
+__device__ __forceinline__ double rcp_approx(double d)
 {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-    double e = fma(-d, r, 1.0);
-    r = fma(r, e, r);
-    e = fma(-d, r, 1.0);
-    return fma(r, e, r);
+    return r;
+}
+
+__device__ __forceinline__ double rcp_step(double d, double r)
+{
+    return fma(r, fma(-d, r, 1.0), r);
+}
+
+__device__ __forceinline__ double rcp_nr(double d)
+{
+    return rcp_step(d, rcp_step(d, rcp_approx(d)));
 }
 
 }  // namespace psb

@@ -17,6 +17,10 @@
 //      [J | dy] on the FP64 tensor cores, tiles of rows bulk-copied into
 //      shared memory and renormalised on the fly.
 //
+// A trial step needs only chi^2 until it is accepted, so it runs a
+// brightness-only form of A and B first (trial_chisq); the full evaluation
+// follows at the accepted parameters.
+//
 // The LM step (damped Gauss-Jordan with full pivoting, accept/reject, lambda
 // update, rms and convergence test) follows Start.cu:300-392, 2838-3021,
 // 4421-4462, 5129-5248 with Numerical-Recipes ia compaction.
@@ -41,15 +45,18 @@ constexpr int kSortCells = kSortBands * kSortSectors;
 constexpr unsigned kWaitLimit = 1u << 24;  // bounded mbarrier waits
 
 // LM scalar slots in shared memory
-enum { S_ALAMDA, S_CHISQ, S_OCHISQ, S_ITERDIFF, S_DEVOLD, S_DEVNEW, S_CHCK, S_AREA, S_TRIAL, S_PIVINV, S_NSCAL };
+enum { S_ALAMDA, S_CHISQ, S_OCHISQ, S_ITERDIFF, S_DEVOLD, S_DEVNEW, S_CHCK, S_AREA, S_TRIAL, S_PIVINV,
+       S_MOM,                        // [3] sum of area-weighted normals at the last trial parameters
+       S_NSCAL = S_MOM + 3 };
 enum { C_ITEM, C_NITER, C_STATUS, C_GJROW0, C_GO, C_TIMEOUT,
        C_YUSE,                       // [kStages] completed uses of each chunk buffer
        C_REL = C_YUSE + kStages,     // [kStages] warps done with the chunk in each buffer
        C_TUSE = C_REL + kStages,     // [2] completed uses of each J^T W J tile buffer
        C_TREL = C_TUSE + 2,          // [2] warps done with each tile buffer (k-slice mode)
-       C_NCTL = C_TREL + 2 };
+       C_NEXT = C_TREL + 2,          // next 32-point tile of the brightness sweep
+       C_NCTL };
 // per-CTA phase clocks (optional instrumentation)
-enum { T_CURV, T_SORT, T_SWEEP, T_CSTAT, T_TILES, T_PSEUDO, T_SOLVE, T_REST, T_TWAIT, T_TSTAGE, T_TSYRK,
+enum { T_CURV, T_SORT, T_SWEEP, T_CSTAT, T_TILES, T_PSEUDO, T_SOLVE, T_REST, T_TRIAL, T_TSTAGE, T_TSYRK,
        T_NPHASE };
 
 constexpr int kWS = 12;  // row stride (floats) of the mixed-precision weight tile: conflict-free A fragments
@@ -94,6 +101,7 @@ struct Sh {
     int *fidx;        // [kMaxFit]
     int *ctl;         // [C_NCTL]
     int ld, mfp, tr;
+    size_t un_bytes;  // size of the storage T, TW, raw, recb and ybuf share
 };
 
 __device__ __forceinline__ double4 ldg4(const double4 *p)
@@ -238,6 +246,7 @@ __host__ __device__ inline size_t carve_bytes(int n_fac, int mfit, int ncp, int 
         s->F = (double4 *)F; s->cone = (float4 *)cone; s->alpha = (double *)alpha; s->covar = (double *)covar;
         s->beta = (double *)beta; s->da = (double *)da; s->a = (double *)a; s->atry = (double *)atry;
         s->T = (double *)un;
+        s->un_bytes = tiles > chunks ? tiles : chunks;
         s->TW = (double *)(un + tsz);
         s->raw = (double *)(un + 2 * tsz);
         s->recb = (double4 *)(un + 2 * tsz + 2 * rsz);
@@ -375,18 +384,20 @@ static __device__ void set_invariants(const DevObject &o, const DevParams &p, co
 // ---------------------------------------------------------------- phase B
 
 // Body-frame geometry of one point: T = Rz(phi) B(beta', lambda) applied to the
-// observer and Sun directions, and (full = true) the derivatives of those
-// vectors w.r.t. beta', lambda, omega plus the phase-function terms
+// observer and Sun directions (kGeoDirections), with the phase function
+// (kGeoScale) and with the derivatives of those vectors w.r.t. beta', lambda,
+// omega and the phase-function derivative terms (kGeoFull)
 // (curve1_point_geometry, Start.cu:2095-2195; ps_phase_mod2pi, Start.cu:687-692).
 // B and its derivatives are read from shared memory through volatile loads so
 // the compiler cannot keep them live in registers across the facet sweep.
+enum { kGeoDirections, kGeoScale, kGeoFull };
 struct PointGeo {
     double e[3], e0[3];
     double db[3], d0b[3], dl[3], d0l[3], dw[2], d0w[2];
     double scale, ff, d2, alph;
 };
 
-template <bool FULL>
+template <int MODE>
 __device__ __forceinline__ void point_geometry(const double *inv, double t, const double *ee,
                                                const double *es, PointGeo &g)
 {
@@ -407,12 +418,14 @@ __device__ __forceinline__ void point_geometry(const double *inv, double t, cons
         g.e[i] = Ti[0] * ee[0] + Ti[1] * ee[1] + Ti[2] * ee[2];
         g.e0[i] = Ti[0] * es[0] + Ti[1] * es[1] + Ti[2] * es[2];
     }
-    if (!FULL) return;
+    if (MODE == kGeoDirections) return;
     const double A = v[2], rD = v[3], K = v[4];
     double cdot = ((ee[0] * es[0]) + ee[1] * es[1]) + ee[2] * es[2];
     g.alph = acos(fmin(1.0, fmax(-1.0, cdot)));
     g.ff = exp2(-1.44269504088896 * (g.alph * rD));
-    g.scale = 1.0 + A * g.ff + K * g.alph;
+    // roundings spelled out: both modes must give the same bits
+    g.scale = __fma_rn(K, g.alph, __dadd_rn(1.0, __dmul_rn(A, g.ff)));
+    if (MODE == kGeoScale) return;
     g.d2 = A * g.ff * g.alph * (rD * rD);
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
@@ -458,7 +471,7 @@ static __device__ void sort_points(const DevObject &o, const Sh &s, int *perm, i
         const double4 pb = ldg4(&o.pt_b[q]);
         const double ee[3] = {pa.y, pa.z, pa.w}, es[3] = {pb.x, pb.y, pb.z};
         PointGeo g;
-        point_geometry<false>(s.inv, pa.x, ee, es, g);
+        point_geometry<kGeoDirections>(s.inv, pa.x, ee, es, g);
         const double bx = g.e[0] + g.e0[0], by = g.e[1] + g.e0[1], bz = g.e[2] + g.e0[2];
         const double n = sqrt(bx * bx + by * by + bz * bz);
         const double cz = n > 0 ? bz / n : 0.0;
@@ -511,6 +524,41 @@ __device__ __forceinline__ void dmma_8x8x4(double &d0, double &d1, double a, dou
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
                  : "+d"(d0), "+d"(d1)
                  : "d"(a), "d"(b));
+}
+
+// Cosine of a direction against a facet normal, and the Lambert +
+// Lommel-Seeliger law mu mu0 (cl + cls / (mu + mu0)) with r = 1 / (mu + mu0).
+// The roundings are spelled out because two sweeps must agree bit for bit:
+// the full one below and the brightness-only one of the trial steps.
+__device__ __forceinline__ double facet_cos(double ex, double ey, double ez, const double4 &f)
+{
+    return __fma_rn(ez, f.z, __fma_rn(ex, f.x, __dmul_rn(ey, f.y)));
+}
+
+__device__ __forceinline__ double facet_scatter(double mu, double mu0, double cl, double cls, double r)
+{
+    return __dmul_rn(__dmul_rn(mu, mu0), __fma_rn(cls, r, cl));
+}
+
+// The 4-facet groups (of up to kMaxChunkGroups, nfc facets) that some lane of
+// the warp may see: the bounding-cone test of facet_cones in FP32, necessary
+// for visibility.  Groups it rules out would add exact zeros.
+__device__ __forceinline__ unsigned group_mask(const float4 *cone, int nfc, bool act, float ex, float ey, float ez,
+                                               float sx, float sy, float sz)
+{
+    unsigned m = 0;
+    if (act) {
+#pragma unroll
+        for (int q = 0; q < kMaxChunkGroups; ++q) {
+            if (4 * q < nfc) {
+                const float4 cn = cone[q];
+                const float ce = fmaf(ez, cn.z, fmaf(ey, cn.y, ex * cn.x));
+                const float c0 = fmaf(sz, cn.z, fmaf(sy, cn.y, sx * cn.x));
+                if (ce > -cn.w && c0 > -cn.w) m |= 1u << q;
+            }
+        }
+    }
+    return __reduce_or_sync(0xffffffffu, m);
 }
 
 // The facet sweep is a kStages-deep pipeline of basis chunks (chunk_facets
@@ -574,7 +622,7 @@ __device__ void brightness_rows(const DevObject &o, const Sh &s, double *rows, c
             const double4 pb = ldg4(&o.pt_b[p]);
             const double ee[3] = {pa.y, pa.z, pa.w}, es[3] = {pb.x, pb.y, pb.z};
             PointGeo geo;
-            point_geometry<false>(s.inv, pa.x, ee, es, geo);
+            point_geometry<kGeoDirections>(s.inv, pa.x, ee, es, geo);
             ex = geo.e[0]; ey = geo.e[1]; ez = geo.e[2];
             sx = geo.e0[0]; sy = geo.e0[1]; sz = geo.e0[2];
         }
@@ -599,23 +647,23 @@ __device__ void brightness_rows(const DevObject &o, const Sh &s, double *rows, c
             for (int q = 0; q < 4; ++q) {
                 const bool inside = k0 + q < nfc;
                 fr[q] = s.F[f0 + (inside ? k0 + q : 0)];
-                mu[q] = ex * fr[q].x + ey * fr[q].y + ez * fr[q].z;
-                mu0[q] = sx * fr[q].x + sy * fr[q].y + sz * fr[q].z;
+                mu[q] = facet_cos(ex, ey, ez, fr[q]);
+                mu0[q] = facet_cos(sx, sy, sz, fr[q]);
                 vis[q] = act && inside && (mu[q] > kTiny) && (mu0[q] > kTiny);
             }
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const double ar = vis[q] ? fr[q].w : 0.0;
                 const double r = rcp_nr(vis[q] ? mu[q] + mu0[q] : 1.0);
-                const double sv = mu[q] * mu0[q] * (cl + cls * r);
+                const double sv = facet_scatter(mu[q], mu0[q], cl, cls, r);
                 const double q0 = mu0[q] * r, q1 = mu[q] * r;
                 const double dsmu = cls * (q0 * q0) + cl * mu0[q];
                 const double dsmu0 = cls * (q1 * q1) + cl * mu[q];
                 const double amm = ar * mu[q] * mu0[q];
-                const double w = ar * sv;
+                const double w = __dmul_rn(ar, sv);
                 const double gg = ar * dsmu;
                 const double g0 = ar * dsmu0;
-                br += w;
+                br = __dadd_rn(br, w);
                 u0 = fma(gg, fr[q].x, u0);
                 u1 = fma(gg, fr[q].y, u1);
                 u2 = fma(gg, fr[q].z, u2);
@@ -670,22 +718,8 @@ __device__ void brightness_rows(const DevObject &o, const Sh &s, double *rows, c
                 // the chunk's 4-facet groups that some lane may see: a bounding-cone
                 // test per group in FP32 (necessary for visibility, see facet_cones);
                 // the groups it rules out would add exact zeros
-                unsigned gmask = 0;
-                if (act) {
-                    const float ex32 = (float)ex, ey32 = (float)ey, ez32 = (float)ez;
-                    const float sx32 = (float)sx, sy32 = (float)sy, sz32 = (float)sz;
-                    const float4 *cg = s.cone + (f0 >> 2);
-#pragma unroll
-                    for (int q = 0; q < kMaxChunkGroups; ++q) {
-                        if (4 * q < nfc) {
-                            const float4 cn = cg[q];
-                            const float ce = fmaf(ez32, cn.z, fmaf(ey32, cn.y, ex32 * cn.x));
-                            const float c0 = fmaf(sz32, cn.z, fmaf(sy32, cn.y, sx32 * cn.x));
-                            if (ce > -cn.w && c0 > -cn.w) gmask |= 1u << q;
-                        }
-                    }
-                }
-                gmask = __reduce_or_sync(0xffffffffu, gmask);
+                unsigned gmask = group_mask(s.cone + (f0 >> 2), nfc, act, (float)ex, (float)ey, (float)ez, (float)sx,
+                                            (float)sy, (float)sz);
                 // Software pipeline over the chunk's groups: the facet terms of
                 // group k0 and the tensor-core step of the group before it (A
                 // fragments already in registers) form one branch-free stretch, so
@@ -726,7 +760,7 @@ __device__ void brightness_rows(const DevObject &o, const Sh &s, double *rows, c
             const double4 pb = ldg4(&o.pt_b[p]);
             const double ee[3] = {pa.y, pa.z, pa.w}, es[3] = {pb.x, pb.y, pb.z};
             PointGeo geo;
-            point_geometry<true>(s.inv, pa.x, ee, es, geo);
+            point_geometry<kGeoFull>(s.inv, pa.x, ee, es, geo);
             const double t1 = (geo.db[0] * u0 + geo.db[1] * u1 + geo.db[2] * u2) +
                               (geo.d0b[0] * w0 + geo.d0b[1] * w1 + geo.d0b[2] * w2);
             const double t2 = (geo.dl[0] * u0 + geo.dl[1] * u1 + geo.dl[2] * u2) +
@@ -786,6 +820,18 @@ __device__ __forceinline__ uint32_t tf32_rna(float x)
     uint32_t r;
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
     return r;
+}
+
+// The mixed sweep's facet cosine and weight (z = a mu mu0, zr = z / (mu + mu0)),
+// shared by the full and the brightness-only form like the FP64 ones above.
+__device__ __forceinline__ float facet_cos(float ex, float ey, float ez, const float4 &f)
+{
+    return __fmaf_rn(ez, f.z, __fmaf_rn(ex, f.x, __fmul_rn(ey, f.y)));
+}
+
+__device__ __forceinline__ float facet_weight(float z, float zr, float cl, float cls)
+{
+    return fmaf(cls, zr, __fmul_rn(cl, z));
 }
 
 // FP32 reciprocal: the special-function unit's approximation refined by one
@@ -860,7 +906,7 @@ __device__ void brightness_rows_mixed(const DevObject &o, const Sh &s, double *r
             const double4 pb = ldg4(&o.pt_b[p]);
             const double ee[3] = {pa.y, pa.z, pa.w}, es[3] = {pb.x, pb.y, pb.z};
             PointGeo geo;
-            point_geometry<false>(s.inv, pa.x, ee, es, geo);
+            point_geometry<kGeoDirections>(s.inv, pa.x, ee, es, geo);
             ex = (float)geo.e[0]; ey = (float)geo.e[1]; ez = (float)geo.e[2];
             sx = (float)geo.e0[0]; sy = (float)geo.e0[1]; sz = (float)geo.e0[2];
         }
@@ -891,8 +937,8 @@ __device__ void brightness_rows_mixed(const DevObject &o, const Sh &s, double *r
                     for (int q = 0; q < 8; ++q) {
                         const bool inside = k0 + q < nfc;
                         const float4 fr = s.F32[f0 + (inside ? k0 + q : 0)];
-                        mu[q] = ex * fr.x + ey * fr.y + ez * fr.z;
-                        mu0[q] = sx * fr.x + sy * fr.y + sz * fr.z;
+                        mu[q] = facet_cos(ex, ey, ez, fr);
+                        mu0[q] = facet_cos(sx, sy, sz, fr);
                         vis[q] = act && inside && (mu[q] > (float)kTiny) && (mu0[q] > (float)kTiny);
                         v8 = v8 || vis[q];
                     }
@@ -914,7 +960,7 @@ __device__ void brightness_rows_mixed(const DevObject &o, const Sh &s, double *r
                         const float r = rcp_f32(vis[q] ? mu[q] + mu0[q] : 1.0f);
                         const float z = fr.w * (mv * m0v);
                         const float zr = z * r;
-                        const float w = fmaf(cls, zr, cl * z);
+                        const float w = facet_weight(z, zr, cl, cls);
                         const float y = ls.y * r;
                         const float gg = m0v * fmaf(y * m0v, r, ls.x);
                         const float g0 = mv * fmaf(y * mv, r, ls.x);
@@ -992,7 +1038,7 @@ __device__ void brightness_rows_mixed(const DevObject &o, const Sh &s, double *r
             const double4 pb = ldg4(&o.pt_b[p]);
             const double ee[3] = {pa.y, pa.z, pa.w}, es[3] = {pb.x, pb.y, pb.z};
             PointGeo geo;
-            point_geometry<true>(s.inv, pa.x, ee, es, geo);
+            point_geometry<kGeoFull>(s.inv, pa.x, ee, es, geo);
             const double br = S64[0], u0 = S64[1], u1 = S64[2], u2 = S64[3];
             const double w0 = S64[4], w1 = S64[5], w2 = S64[6], t4 = S64[7], t5 = S64[8];
             const double t1 = (geo.db[0] * u0 + geo.db[1] * u1 + geo.db[2] * u2) +
@@ -1073,11 +1119,16 @@ struct SyrkAcc {
     int bj[kMaxBlk], bk[kMaxBlk], nblk;   // block mode
 };
 
+__device__ __forceinline__ bool syrk_slices(int mfit, int tile_rows)
+{
+    return fit_mpad(mfit) <= 64 && tile_rows == 4 * kWarps;
+}
+
 __device__ __forceinline__ void syrk_init(int mfit, int tile_rows, SyrkAcc &acc)
 {
     const int warp = threadIdx.x >> 5;
     acc.nb = fit_mpad(mfit) / 8;
-    acc.slice = (acc.nb <= 8 && tile_rows == 4 * kWarps) ? 1 : 0;
+    acc.slice = syrk_slices(mfit, tile_rows) ? 1 : 0;
     const int nblocks = acc.nb * (acc.nb + 1) / 2;
     acc.nblk = 0;
 #pragma unroll
@@ -1193,19 +1244,28 @@ __device__ __forceinline__ void syrk_store(const Sh &s, int mfit, const SyrkAcc 
     __syncthreads();
 }
 
-// One full evaluation (mrqcof) at parameter vector a in shared memory.
-// Writes alpha (symmetric, stride ld) to dst, beta to dvec; returns chi^2 to
-// every thread.
-template <int NCP, bool MIXED>
-__device__ double evaluate(const DevObject &o, const DevParams &p, const Sh &s, const double *a,
-                           double *dst, double *dvec, double *rows, double *cstat, int *perm, double conw_r)
+// Sum of the area-weighted normals at the current facet areas, to every thread.
+static __device__ void moment_sums(const DevObject &o, const Sh &s, double (&r)[3])
 {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int ma = o.ma, mfit = o.mfit, mfp = s.mfp, RS = o.row_stride, CS = ma + 3;
+    r[0] = r[1] = r[2] = 0;
+    for (int fi = threadIdx.x; fi < o.n_fac; fi += kThreads) {
+        const double4 fr = s.F[fi];
+        r[0] += fr.w * fr.x;
+        r[1] += fr.w * fr.y;
+        r[2] += fr.w * fr.z;
+    }
+    block_sum<3>(r, s.red);
+}
 
-    if (o.cstat_smem) cstat = s.cst;  // stride ma + 3 fits inside rs + 2
-    tmark(p, s, T_REST);
-    double area_sum = shape_areas(o, s, a);
+// What an evaluation at parameter vector a starts with: facet areas, their
+// sum (S_AREA), the invariants, in mixed precision the FP32 facet tables, and
+// the point order.
+template <bool MIXED>
+static __device__ void evaluation_setup(const DevObject &o, const DevParams &p, const Sh &s, const double *a, int *perm)
+{
+    const int tid = threadIdx.x;
+    if (tid == 0) s.ctl[C_NEXT] = 0;
+    const double area_sum = shape_areas(o, s, a);
     if (tid == 0) s.scal[S_AREA] = area_sum;
     set_invariants(o, p, s, a);
     if constexpr (MIXED) {  // FP32 facet tables of the mixed-precision sweep
@@ -1218,9 +1278,269 @@ __device__ double evaluate(const DevObject &o, const DevParams &p, const Sh &s, 
         __syncthreads();
     }
     tmark(p, s, T_CURV);
-
     sort_points(o, s, perm, perm + o.n_points);
     tmark(p, s, T_SORT);
+}
+
+// 1 / sum(ymod) and the renormalisation coefficient of relative curve c.
+__device__ __forceinline__ void renormalise_curve(const DevObject &o, const Sh &s, int c, double sum)
+{
+    const double rave = 1.0 / sum;
+    s.crave[c] = rave;
+    s.ccoef[c] = o.curve_sig[c] * (o.curve_start[c + 1] - o.curve_start[c]) * rave;
+}
+
+// ---------------------------------------------------------------- trial steps
+
+// Raw model brightness of all points (column ma of the full sweep's rows, bit
+// for bit) into ym: the same facets in the same order with the same roundings,
+// without the derivative sums and the basis.  About 18 FP64 operations per
+// (point, facet) instead of 39 and a rank-1 update of n_coef columns, no
+// accumulator file, and no basis traffic; warps take 32-point tiles from a
+// counter.  What bounds it: the FP64 pipe and, with two warps per scheduler,
+// the latency of its chains (pipe 63 % busy); 8 facets a step are in flight
+// per lane, their stages written side by side.  Visibility by integer
+// comparison of the bit patterns, which spares the FP64 pipe two operations a
+// facet, was 6 % slower: the integer instructions cost more issue slots.
+template <bool MIXED>
+static __device__ void brightness_only(const DevObject &o, const Sh &s, double *ym, const int *perm)
+{
+    const int lane = threadIdx.x & 31;
+    const int np = o.n_points, nf = o.n_fac, ntiles = (np + 31) / 32;
+    const double cl = s.inv[5], cls = s.inv[6];
+    for (;;) {
+        int tile = 0;
+        if (lane == 0) tile = atomicAdd(&s.ctl[C_NEXT], 1);
+        tile = __shfl_sync(0xffffffffu, tile, 0);
+        if (tile >= ntiles) break;
+        const int idx = tile * 32 + lane;
+        const bool act = idx < np;
+        const int p = perm[min(idx, np - 1)];
+        PointGeo geo;
+        {
+            const double4 pa = ldg4(&o.pt_a[p]);
+            const double4 pb = ldg4(&o.pt_b[p]);
+            const double ee[3] = {pa.y, pa.z, pa.w}, es[3] = {pb.x, pb.y, pb.z};
+            point_geometry<kGeoScale>(s.inv, pa.x, ee, es, geo);
+        }
+        // a lane past the last point sees no facet
+        const double ex = act ? geo.e[0] : 0.0, ey = act ? geo.e[1] : 0.0, ez = act ? geo.e[2] : 0.0;
+        const double sx = geo.e0[0], sy = geo.e0[1], sz = geo.e0[2];
+        const float ex32 = (float)ex, ey32 = (float)ey, ez32 = (float)ez;
+        const float sx32 = (float)sx, sy32 = (float)sy, sz32 = (float)sz;
+        // groups of 4 facets that some lane may see, 32 groups a mask word
+        auto groups = [&](int g0, int ng) {
+            unsigned m = 0;
+#pragma unroll 8
+            for (int q = 0; q < min(32, ng - g0); ++q) {
+                const float4 cn = s.cone[g0 + q];
+                const float ce = fmaf(ez32, cn.z, fmaf(ey32, cn.y, ex32 * cn.x));
+                const float c0 = fmaf(sz32, cn.z, fmaf(sy32, cn.y, sx32 * cn.x));
+                if (ce > -cn.w && c0 > -cn.w) m |= 1u << q;
+            }
+            return __reduce_or_sync(0xffffffffu, act ? m : 0u);
+        };
+        double br = 0;
+        if constexpr (MIXED) {
+            // steps of 8 facets, each summed in FP32 and flushed to FP64
+            const float clf = (float)cl, clsf = (float)cls;
+            auto weight = [&](const float4 &fr) {
+                const float mu = facet_cos(ex32, ey32, ez32, fr), mu0 = facet_cos(sx32, sy32, sz32, fr);
+                const bool vis = mu > (float)kTiny && mu0 > (float)kTiny;
+                const float z = __fmul_rn(fr.w, __fmul_rn(mu, mu0));
+                const float w = facet_weight(z, __fmul_rn(z, rcp_f32(mu + mu0)), clf, clsf);
+                return vis ? w : 0.0f;
+            };
+            const int ng = 2 * (nf >> 3);
+            for (int g0 = 0; g0 < ng; g0 += 32) {
+                unsigned m = groups(g0, ng);
+                m = (m | m >> 1) & 0x55555555u;
+#pragma unroll 1
+                while (m) {
+                    const float4 *F = s.F32 + 4 * (g0 + __ffs(m) - 1);
+                    m &= m - 1;
+                    float w[8], sum = 0.0f;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) w[q] = weight(F[q]);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) sum = __fadd_rn(sum, w[q]);
+                    br += (double)sum;
+                }
+            }
+            if (nf & 7) {
+                float sum = 0.0f;
+                for (int f = nf & ~7; f < nf; ++f) sum = __fadd_rn(sum, weight(s.F32[f]));
+                br += (double)sum;
+            }
+        } else {
+            // N facets, stage by stage so that their chains interleave
+            auto add = [&](auto n, const double4 *F0, const double4 *F1) {
+                constexpr int N = decltype(n)::value;
+                double mu[N], mu0[N], ar[N], r[N], d[N];
+#pragma unroll
+                for (int q = 0; q < N; ++q) {
+                    const double4 fr = q < 4 ? F0[q] : F1[q - 4];
+                    mu[q] = facet_cos(ex, ey, ez, fr);
+                    mu0[q] = facet_cos(sx, sy, sz, fr);
+                    ar[q] = fr.w;
+                }
+#pragma unroll
+                for (int q = 0; q < N; ++q) {
+                    d[q] = mu[q] + mu0[q];
+                    r[q] = rcp_approx(d[q]);
+                }
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+#pragma unroll
+                    for (int q = 0; q < N; ++q) r[q] = rcp_step(d[q], r[q]);
+                }
+#pragma unroll
+                for (int q = 0; q < N; ++q) {
+                    const double w = __dmul_rn(ar[q], facet_scatter(mu[q], mu0[q], cl, cls, r[q]));
+                    d[q] = mu[q] > kTiny && mu0[q] > kTiny ? w : 0.0;
+                }
+#pragma unroll
+                for (int q = 0; q < N; ++q) br = __dadd_rn(br, d[q]);
+            };
+            const int ng = nf >> 2;
+            for (int g0 = 0; g0 < ng; g0 += 32) {
+                unsigned m = groups(g0, ng);
+#pragma unroll 1
+                while (m) {
+                    // two groups a step while there are two, added in facet order
+                    const double4 *F0 = s.F + 4 * (g0 + __ffs(m) - 1);
+                    m &= m - 1;
+                    if (m) {
+                        const double4 *F1 = s.F + 4 * (g0 + __ffs(m) - 1);
+                        m &= m - 1;
+                        add(std::integral_constant<int, 8>{}, F0, F1);
+                    } else {
+                        add(std::integral_constant<int, 4>{}, F0, F0);
+                    }
+                }
+            }
+            for (int f = nf & ~3; f < nf; ++f) add(std::integral_constant<int, 1>{}, s.F + f, s.F + f);
+        }
+        if (act) ym[p] = __dmul_rn(br, geo.scale);
+    }
+}
+
+// chi^2 alone at the trial parameters s.atry, equal bit for bit to the one the
+// full evaluation there gives: every trial step needs it, but half of the
+// steps and more are rejected, and those need nothing else.  Measured at the
+// production object (3698 points, 512 facets, 49 coefficients):
+//   full evaluation 2.85e6 cycles, this 0.66e6; 53 % of the trial steps of
+//   its 50-iteration fits are rejected.  One wave of 50-iteration fits went
+//   from 77.9 to 57.6 ms (310 fits: 234 -> 170 ms).
+// Leaves the facet areas (s.F), the invariants (s.inv) and the point order
+// (perm) of the trial parameters for the full evaluation that follows an
+// accepted step, the summed area in S_AREA and the summed area-weighted
+// normals in S_MOM.  All threads must call it.
+template <bool MIXED>
+static __device__ double trial_chisq(const DevObject &o, const DevParams &p, const Sh &s, double *rows, int *perm,
+                                     double conw_r)
+{
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int np = o.n_points, mfit = o.mfit;
+    tmark(p, s, T_REST);
+    evaluation_setup<MIXED>(o, p, s, s.atry, perm);
+
+    // per point: model brightness, then residual and weighted residual -- in
+    // the idle tile storage if they fit there, else in the row slab
+    double *dy = 2 * sizeof(double) * (size_t)np <= s.un_bytes ? s.ybuf : rows;
+    double *dyw = dy + np;
+    brightness_only<MIXED>(o, s, dy, perm);
+    __syncthreads();
+    tmark(p, s, T_TRIAL);
+    // renormalisation of the relative curves: one thread per curve adds its
+    // points in order
+    for (int c = tid; c < o.n_curves; c += kThreads) {
+        if (!o.curve_rel[c]) continue;
+        const int p0 = o.curve_start[c], p1 = o.curve_start[c + 1];
+        double sum = 0;
+        constexpr int kAhead = 8;
+        for (int q0 = p0; q0 < p1; q0 += kAhead) {
+            double v[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) v[u] = q0 + u < p1 ? dy[q0 + u] : 0.0;
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) sum += v[u];
+        }
+        renormalise_curve(o, s, c, sum);
+    }
+    // area-weighted normals: the pseudo-points' residuals
+    double ym[3];
+    moment_sums(o, s, ym);  // its barriers also order the coefficients above
+    if (tid == 0)
+        for (int i = 0; i < 3; ++i) s.scal[S_MOM + i] = ym[i];
+    for (int q = tid; q < np; q += kThreads) {
+        const double4 rec = ldg4(&o.pt_rec[q]);
+        double ymod = dy[q];
+        if (rec.w != 0.0) ymod = __dmul_rn(s.ccoef[(int)rec.z], ymod);
+        const double d = __dsub_rn(rec.x, ymod);
+        dy[q] = d;
+        dyw[q] = __dmul_rn(d, rec.y);
+    }
+    __syncthreads();
+
+    // chi^2 as the full evaluation's tensor-core update forms it: element
+    // (mfit, mfit) of the augmented matrix, the same MMA steps in the same
+    // order with every other column zero.  k-slice mode: warp w adds rows
+    // 4w..4w+3 of every 32; block mode: the warp that owns the last block
+    // adds 4 rows a step.  The pseudo-points come last.
+    const int nb = fit_mpad(mfit) / 8;
+    const bool slice = syrk_slices(mfit, s.tr);
+    const int owner = slice ? 0 : (nb * (nb + 1) / 2 - 1) & (kWarps - 1);
+    const int m = mfit & 7, k = lane & 3;
+    const bool col = (lane >> 2) == m;
+    double c0 = 0.0, c1 = 0.0;
+    if (slice || warp == owner) {
+        const int step = slice ? 4 * kWarps : 4;
+        constexpr int kAhead = 8;
+        for (int q0 = (slice ? 4 * warp : 0); q0 < ((np + step - 1) / step) * step; q0 += kAhead * step) {
+            double fa[kAhead], fb[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                const int q = q0 + u * step + k;
+                const bool in = col && q < np;
+                fa[u] = in ? dyw[q] : 0.0;
+                fb[u] = in ? dy[q] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) dmma_8x8x4(c0, c1, fa[u], fb[u]);
+        }
+        if (warp == owner) {
+            const double d = (col && k < 3) ? 0.0 - (k == 0 ? ym[0] : k == 1 ? ym[1] : ym[2]) : 0.0;
+            dmma_8x8x4(c0, c1, __dmul_rn(d, __dmul_rn(conw_r, conw_r)), d);
+        }
+        if (lane == 4 * m + (m >> 1)) s.red[warp] = (m & 1) ? c1 : c0;
+    }
+    __syncthreads();
+    double chisq = 0.0;
+    if (slice)
+        for (int w = 0; w < kWarps; ++w) chisq += s.red[w];
+    else
+        chisq = s.red[owner];
+    __syncthreads();
+    tmark(p, s, T_REST);
+    return chisq;
+}
+
+// One full evaluation (mrqcof) at parameter vector a in shared memory; ready:
+// trial_chisq has just run at the same parameters and its areas, invariants
+// and point order still stand.
+// Writes alpha (symmetric, stride ld) to dst, beta to dvec; returns chi^2 to
+// every thread.
+template <int NCP, bool MIXED>
+__device__ double evaluate(const DevObject &o, const DevParams &p, const Sh &s, const double *a, bool ready,
+                           double *dst, double *dvec, double *rows, double *cstat, int *perm, double conw_r)
+{
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int ma = o.ma, mfit = o.mfit, mfp = s.mfp, RS = o.row_stride, CS = ma + 3;
+
+    if (o.cstat_smem) cstat = s.cst;  // stride ma + 3 fits inside rs + 2
+    tmark(p, s, T_REST);
+    if (!ready) evaluation_setup<MIXED>(o, p, s, a, perm);
     if constexpr (MIXED)
         brightness_rows_mixed<NCP>(o, s, rows, perm);
     else
@@ -1260,12 +1580,7 @@ __device__ double evaluate(const DevObject &o, const DevParams &p, const Sh &s, 
             if (lane + 32 * j <= ma) cstat[(size_t)c * CS + lane + 32 * j] = sum[j];
         __syncwarp();
         if (lane == 0) {
-            const double rave = 1.0 / cstat[(size_t)c * CS + ma];
-            const double coef = o.curve_sig[c] * (p1 - p0) * rave;
-            cstat[(size_t)c * CS + ma + 1] = rave;
-            cstat[(size_t)c * CS + ma + 2] = coef;
-            s.crave[c] = rave;
-            s.ccoef[c] = coef;
+            renormalise_curve(o, s, c, cstat[(size_t)c * CS + ma]);
         }
     }
     __syncthreads();
@@ -1391,7 +1706,6 @@ __device__ double evaluate(const DevObject &o, const DevParams &p, const Sh &s, 
         const int b = t & 1, r0 = t * TR, nrows = min(TR, np - r0);
         tmark(p, s, T_TILES);
         if (!mbar_wait(&s.tbar[b], (uint32_t)((s.ctl[C_TUSE + b] + (t >> 1)) & 1))) timeout = true;
-        tmark(p, s, T_TWAIT);
         const double *rb = s.raw + (size_t)b * TR * RS;
         const double4 *rc = s.recb + b * TR;
         // per-row scalars: lane k < rpw computes row warp * rpw + k
@@ -1462,14 +1776,8 @@ __device__ double evaluate(const DevObject &o, const DevParams &p, const Sh &s, 
     // convexity regularisation pseudo-points (mrqcof_curve1_last_opt, Start.cu:2539-2612)
     {
         const int nc = o.n_coef, nf = o.n_fac;
-        double ym[3] = {0, 0, 0};
-        for (int fi = tid; fi < nf; fi += kThreads) {
-            const double4 fr = s.F[fi];
-            ym[0] += fr.w * fr.x;
-            ym[1] += fr.w * fr.y;
-            ym[2] += fr.w * fr.z;
-        }
-        block_sum<3>(ym, s.red);
+        double ym[3];
+        moment_sums(o, s, ym);
         // raw derivative d ym_i / d a_k for shape coefficient k = tid: groups
         // of nc threads take consecutive facet ranges, their partial sums
         // (staged in the idle tile buffer) are added in group order
@@ -1846,6 +2154,7 @@ __device__ __forceinline__ void fit_one(const DevObject &o, const DevParams &p, 
     }
     __syncthreads();
 
+    bool moved = false;  // the last trial step was accepted: alpha and beta are the previous parameters'
     for (;;) {
         // convergence test (CudaCalculateIter1Begin, Start.cu:4421-4462)
         if (tid == 0) {
@@ -1857,11 +2166,18 @@ __device__ __forceinline__ void fit_one(const DevObject &o, const DevParams &p, 
         if (!s.ctl[C_GO]) break;
         const bool first = s.scal[S_ALAMDA] < 0;
         __syncthreads();
-        if (first) {
-            if (tid == 0) s.scal[S_ALAMDA] = p.alamda_start;
-            double oc = evaluate<NCP, MIXED>(o, p, s, s.a, s.alpha, s.beta, rows, cstat, perm, p.conw_r);
-            if (tid == 0) s.scal[S_OCHISQ] = oc;
-            for (int q = tid; q <= ma; q += kThreads) s.atry[q] = s.a[q];
+        // alpha and beta at the current parameters: at the start, and after an
+        // accepted step -- only now, so a fit that ends with one does without
+        if (first || moved) {
+            const double oc = evaluate<NCP, MIXED>(o, p, s, s.a, moved, s.alpha, s.beta, rows, cstat, perm, p.conw_r);
+            moved = false;
+            if (first) {
+                if (tid == 0) {
+                    s.scal[S_ALAMDA] = p.alamda_start;
+                    s.scal[S_OCHISQ] = oc;
+                }
+                for (int q = tid; q <= ma; q += kThreads) s.atry[q] = s.a[q];
+            }
             __syncthreads();
         }
         // damped normal matrix and solve (mrqmin_1_end_opt)
@@ -1882,14 +2198,13 @@ __device__ __forceinline__ void fit_one(const DevObject &o, const DevParams &p, 
             if (err == 2 && tid == 0) s.ctl[C_STATUS] |= kStatusSingular;
         }
         __syncthreads();
-        const double chisq = evaluate<NCP, MIXED>(o, p, s, s.atry, s.covar, s.da, rows, cstat, perm, p.conw_r);
+        const double chisq = trial_chisq<MIXED>(o, p, s, rows, perm, p.conw_r);
         // accept / reject (mrqmin_2_end, Start.cu:300-392)
         const bool accept = chisq < s.scal[S_OCHISQ];
         __syncthreads();
         if (accept) {
-            for (int idx = tid; idx < mfit * ld; idx += kThreads) s.alpha[idx] = s.covar[idx];
-            if (tid < mfit) s.beta[tid] = s.da[tid];
             for (int q = tid; q <= ma; q += kThreads) s.a[q] = s.atry[q];
+            moved = true;
         }
         if (tid == 0) {
             if (isnan(chisq)) s.ctl[C_STATUS] |= kStatusNanChisq;
@@ -1908,15 +2223,14 @@ __device__ __forceinline__ void fit_one(const DevObject &o, const DevParams &p, 
         const double ch = s.scal[S_CHISQ];
         if (niter == 1 || ch < s.scal[S_OCHISQ]) {
             __syncthreads();
-            const double area_sum = shape_areas(o, s, s.a);
-            double r[3] = {0, 0, 0};
-            for (int fi = tid; fi < o.n_fac; fi += kThreads) {
-                const double4 fr = s.F[fi];
-                r[0] += fr.w * fr.x;
-                r[1] += fr.w * fr.y;
-                r[2] += fr.w * fr.z;
+            // the areas of an accepted step are the trial's; a rejected first
+            // step goes back to the start parameters'
+            double r[3] = {s.scal[S_MOM], s.scal[S_MOM + 1], s.scal[S_MOM + 2]};
+            double area_sum = s.scal[S_AREA];
+            if (!accept) {
+                area_sum = shape_areas(o, s, s.a);
+                moment_sums(o, s, r);
             }
-            block_sum<3>(r, s.red);
             if (tid == 0) {
                 s.scal[S_OCHISQ] = ch;
                 s.scal[S_AREA] = area_sum;
@@ -2008,7 +2322,7 @@ fit_kernel(DevObject o, DevParams p, const FitItem *items, int n_items, int *que
             int *perm = reinterpret_cast<int *>(rows + scratch_perm(o.n_points, o.row_stride, o.n_curves, ma));
             for (int q = tid; q <= ma; q += kThreads) s.a[q] = ev.a[q];
             __syncthreads();
-            double chisq = evaluate<NCP, MIXED>(o, p, s, s.a, s.alpha, s.beta, rows, cstat, perm, p.conw_r);
+            double chisq = evaluate<NCP, MIXED>(o, p, s, s.a, false, s.alpha, s.beta, rows, cstat, perm, p.conw_r);
             for (int idx = tid; idx < mfit * mfit; idx += kThreads) {
                 const int j = idx / mfit, k = idx - j * mfit;
                 ev.alpha[idx] = s.alpha[j * ld + k];

@@ -315,7 +315,7 @@ class Engine:
         _check(lib().ps_gpu_status(self.h, _p(f, C.c_int32)))
         return int(f[0])
 
-    PHASES = ("curv", "sort", "sweep", "curve_stats", "jtwj_other", "pseudo", "solve", "rest", "tile_wait",
+    PHASES = ("curv", "sort", "sweep", "curve_stats", "jtwj_other", "pseudo", "solve", "rest", "trial",
               "tile_stage", "tile_syrk")
 
     def phase_clocks(self, enable=True):
