@@ -86,10 +86,13 @@ extern "C" void ps_gpu_unprepare(ps_gpu *h)
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
     h->facet.release(); h->pt_a.release(); h->pt_b.release(); h->pt_rec.release();
-    h->ysh.release(); h->ysh32.release(); h->pt_w.release(); h->curve_sig.release(); h->cg_first.release();
+    h->ysh.release(); h->ysh_t.release(); h->ysh32.release(); h->pt_w.release(); h->curve_sig.release(); h->cg_first.release();
     h->scratch.release(); h->eval_buf.release();
     h->pt_curve.release(); h->curve_start.release(); h->curve_rel.release(); h->fidx.release();
     h->queue.release(); h->status.release(); h->items.release(); h->out.release(); h->phase.release();
+    if (h->fork) cudaEventDestroy(h->fork);
+    if (h->join) cudaEventDestroy(h->join);
+    if (h->side) cudaStreamDestroy(h->side);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
 }
@@ -190,6 +193,9 @@ extern "C" ps_status ps_gpu_configure(ps_gpu *h, double freq_start, double freq_
     std::vector<double> ysh((size_t)numfac * ncp, 0.0);
     for (int f = 0; f < numfac; ++f)
         for (int k = 0; k < nc; ++k) ysh[(size_t)f * ncp + k] = shape->d_sphere[(size_t)f * nc + k];
+    std::vector<double> ysh_t((size_t)numfac * nc);
+    for (int k = 0; k < nc; ++k)
+        for (int f = 0; f < numfac; ++f) ysh_t[(size_t)k * numfac + f] = shape->d_sphere[(size_t)f * nc + k];
     // mixed precision: the basis as TF32 high and low parts, chunk by chunk
     // ([chunk][hi | lo][chunk facets][ncp], zero past the last facet)
     std::vector<float> ysh32;
@@ -229,6 +235,7 @@ extern "C" ps_status ps_gpu_configure(ps_gpu *h, double freq_start, double freq_
     cudaStream_t s = h->stream;
     PSB_CUDA(psb::upload(h->facet, facet, s));
     PSB_CUDA(psb::upload(h->ysh, ysh, s));
+    PSB_CUDA(psb::upload(h->ysh_t, ysh_t, s));
     if (mixed) PSB_CUDA(psb::upload(h->ysh32, ysh32, s));
     PSB_CUDA(psb::upload(h->pt_a, pa, s));
     PSB_CUDA(psb::upload(h->pt_b, pb, s));
@@ -240,7 +247,7 @@ extern "C" ps_status ps_gpu_configure(ps_gpu *h, double freq_start, double freq_
     PSB_CUDA(psb::upload(h->curve_sig, csig, s));
     PSB_CUDA(psb::upload(h->fidx, fidx, s));
     PSB_CUDA(psb::upload(h->cg_first, cgf, s));
-    PSB_CUDA(h->queue.ensure(1));
+    PSB_CUDA(h->queue.ensure(2));
     if (!h->status.ptr) {
         PSB_CUDA(h->status.ensure(1));
         PSB_CUDA(cudaMemsetAsync(h->status.ptr, 0, sizeof(int), s));
@@ -260,6 +267,7 @@ extern "C" ps_status ps_gpu_configure(ps_gpu *h, double freq_start, double freq_
     o.cstat_smem = cstat_smem;
     o.facet = h->facet.ptr;
     o.ysh = h->ysh.ptr;
+    o.ysh_t = h->ysh_t.ptr;
     o.pt_a = h->pt_a.ptr;
     o.pt_b = h->pt_b.ptr;
     o.pt_w = h->pt_w.ptr;
@@ -320,14 +328,37 @@ extern "C" ps_status ps_gpu_occupancy(ps_gpu *h, int32_t *ctas_per_sm, int32_t *
     return PS_OK;
 }
 
-// Enqueues the fit kernel over n device-resident items.
+// Enqueues the fit kernel over n device-resident items: whole waves by single
+// CTAs, what is left by teams beside them.
 static ps_status enqueue_fits(ps_gpu *h, int n, const psb::FitItem *d_items, psb::FitOut *d_out)
 {
-    const int n_ctas = std::max(1, std::min(n, h->ctas_per_sm * h->n_sm));
-    PSB_CUDA(h->scratch.ensure(h->scratch_per_cta * (size_t)n_ctas));
-    PSB_CUDA(cudaMemsetAsync(h->queue.ptr, 0, sizeof(int), h->stream));
-    int e = psb::launch_fits(h->obj, h->prm, d_items, n, h->queue.ptr, d_out, h->scratch.ptr, h->scratch_per_cta,
-                             n_ctas, h->status.ptr, h->stream);
+    const psb::FitPlan pl = psb::plan_fits(h->obj, n, h->ctas_per_sm * h->n_sm, 0, true);
+    PSB_CUDA(h->scratch.ensure(h->scratch_per_cta * (size_t)pl.slabs()));
+    PSB_CUDA(cudaMemsetAsync(h->queue.ptr, 0, 2 * sizeof(int), h->stream));
+    const bool both = pl.main_items > 0 && pl.team_items > 0;
+    cudaStream_t ts = h->stream;
+    if (both) {
+        if (!h->side) {
+            PSB_CUDA(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
+            PSB_CUDA(cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming));
+            PSB_CUDA(cudaEventCreateWithFlags(&h->join, cudaEventDisableTiming));
+        }
+        ts = h->side;
+        PSB_CUDA(cudaEventRecord(h->fork, h->stream));
+        PSB_CUDA(cudaStreamWaitEvent(ts, h->fork, 0));
+    }
+    int e = 0;
+    if (pl.main_items > 0)
+        e = psb::launch_fits(h->obj, h->prm, d_items, pl.main_items, h->queue.ptr, d_out, h->scratch.ptr,
+                             h->scratch_per_cta, pl.main_ctas, h->status.ptr, h->stream);
+    if (!e && pl.team_items > 0)
+        e = psb::launch_fit_teams(h->obj, h->prm, d_items + pl.main_items, pl.team_items, h->queue.ptr + 1,
+                                  d_out + pl.main_items, h->scratch.ptr + h->scratch_per_cta * (size_t)pl.main_ctas,
+                                  h->scratch_per_cta, pl.teams, pl.team_size, h->status.ptr, ts);
+    if (both) {  // joined on the error path too, for a stream under capture
+        PSB_CUDA(cudaEventRecord(h->join, ts));
+        PSB_CUDA(cudaStreamWaitEvent(h->stream, h->join, 0));
+    }
     if (e) return psb_fail_cuda(e, "fit kernel launch");
     return PS_OK;
 }

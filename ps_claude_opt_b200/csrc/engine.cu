@@ -1,6 +1,9 @@
 // engine.cu -- template dispatch and launch wrappers of the fit kernel.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <climits>
+
 #include "engine.h"
 #include "fit_kernel.cuh"
 
@@ -27,6 +30,11 @@ size_t fit_smem_bytes(int n_fac, int mfit, int ncp, int n_curves, int row_stride
     return carve_bytes(n_fac, mfit, ncp, n_curves, row_stride, tile_rows, cstat_smem, mixed, nullptr, nullptr);
 }
 
+static size_t fit_smem_bytes(const DevObject &o)
+{
+    return fit_smem_bytes(o.n_fac, o.mfit, o.ncp, o.n_curves, o.row_stride, o.tile_rows, o.cstat_smem, o.mixed);
+}
+
 int chunk_facets_of(int ncp) { return chunk_facets(ncp); }
 
 size_t fit_scratch_doubles(const DevObject &o)
@@ -49,6 +57,37 @@ PSB_MIXED_LIST(PSB_DECLM)
 #define PSB_DECLB(N) KernelFn fit_kernel_batch_ptr_##N();
 PSB_NCP_LIST(PSB_DECLB)
 #undef PSB_DECLB
+
+#define PSB_DECLT(N) KernelFn fit_kernel_team_ptr_##N();
+PSB_NCP_LIST(PSB_DECLT)
+#undef PSB_DECLT
+#define PSB_DECLMT(N) KernelFn fit_kernel_mixed_team_ptr_##N();
+PSB_MIXED_LIST(PSB_DECLMT)
+#undef PSB_DECLMT
+
+static KernelFn team_kernel_for(int ncp, int mixed)
+{
+    if (mixed) {
+        switch (ncp) {
+#define PSB_CASEMT(N) \
+    case N:           \
+        return fit_kernel_mixed_team_ptr_##N();
+            PSB_MIXED_LIST(PSB_CASEMT)
+#undef PSB_CASEMT
+        default:
+            return nullptr;
+        }
+    }
+    switch (ncp) {
+#define PSB_CASET(N) \
+    case N:          \
+        return fit_kernel_team_ptr_##N();
+        PSB_NCP_LIST(PSB_CASET)
+#undef PSB_CASET
+    default:
+        return nullptr;
+    }
+}
 
 static KernelFn batch_kernel_for(int ncp)
 {
@@ -154,11 +193,114 @@ int launch_fits_batch(const DevObject &env, const DevObject *d_objs, const DevPa
     return (int)cudaGetLastError();
 }
 
+// Launch configuration of `groups` teams of team_size CTAs.
+struct TeamLaunch {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    KernelFn fn = nullptr;
+    int prepare(const DevObject &o, int groups, int team_size, void *stream)
+    {
+        fn = team_kernel_for(o.ncp, o.mixed);
+        if (!fn) return (int)cudaErrorInvalidValue;
+        const size_t smem = fit_smem_bytes(o);
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = team_size;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.gridDim = dim3(groups * team_size);
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = (cudaStream_t)stream;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        return (int)cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    }
+};
+
+// Teams of this size the GPU holds at a time (0 if none).
+static int max_teams(const DevObject &o, int team_size)
+{
+    TeamLaunch l;
+    int n = 0;
+    if (l.prepare(o, 1, team_size, nullptr) != 0) return 0;
+    if (cudaOccupancyMaxActiveClusters(&n, l.fn, &l.cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+
+constexpr int kTeamSizes[3] = {2, 4, 8};
+// Time of one fit by a team, as a share of its time by one CTA.  Measured, FP64,
+// teams of 2 / 4 / 8: production object 0.73 / 0.42 / 0.27, largest models
+// 0.78 / 0.48 / 0.31, config 1 0.91 / 0.64 / 0.45; mixed precision 0.88 / 0.53 /
+// 0.33.  (The solve and the barriers do not divide, and a team's few tiles a
+// warp leave the sweep's rounds uneven.)
+constexpr double kTeamTime[3] = {0.78, 0.46, 0.31};
+
+FitPlan plan_fits(const DevObject &o, int n, int resident, int max_slabs, bool mixable)
+{
+    FitPlan pl;
+    const int slabs = max_slabs > 0 ? max_slabs : INT_MAX;
+    const int wave = std::max(1, std::min(resident, slabs));  // fits one wave of single CTAs holds
+    const int waves = n / wave, rest = n - waves * wave;
+    pl.main_items = n;
+    pl.main_ctas = std::min(n, wave);
+    // with nothing but whole waves, or a last wave too full to split, single
+    // CTAs are best; without a second stream all fits go one way.  A wave of
+    // single CTAs takes 1, so teams must make the rest cheaper: with 148 SMs
+    // teams of 8 up to 18 fits (10 production fits: 57.6 -> 15.9 ms), of 4 up to
+    // about 37 (30 fits: 24.5 ms), of 2 up to 74 (70 fits: 42.5 ms), single CTAs
+    // above (140 fits: 58 ms)
+    const int items = mixable ? rest : n;
+    if (items == 0) return pl;
+    double best = mixable ? 1.0 : (n + wave - 1) / wave;
+    best *= 0.95;
+    for (int k = 0; k < 3; ++k) {
+        // teams that this number of fits could use at once
+        if (mixable && (double)((items * kTeamSizes[k] + resident - 1) / resident) * kTeamTime[k] >= best) continue;
+        const int teams = std::min({max_teams(o, kTeamSizes[k]), slabs, items});
+        if (teams < 1) continue;
+        const double t = ((items + teams - 1) / teams) * kTeamTime[k];
+        if (t < best) {
+            best = t;
+            pl.teams = teams;
+            pl.team_size = kTeamSizes[k];
+        }
+    }
+    if (pl.teams) {
+        pl.team_items = items;
+        pl.main_items = n - items;
+        pl.main_ctas = std::min(pl.main_items, wave);
+    }
+    return pl;
+}
+
+int launch_fit_teams(const DevObject &o, const DevParams &p, const FitItem *items, int n_items, int *queue,
+                     FitOut *out, double *scratch, size_t scratch_per_cta, int groups, int team_size, int *status,
+                     void *stream)
+{
+    TeamLaunch l;
+    const int e = l.prepare(o, groups, team_size, stream);
+    if (e) return e;
+    EvalOut ev{};
+    return (int)cudaLaunchKernelEx(&l.cfg, l.fn, o, p, items, n_items, queue, out, scratch, scratch_per_cta, status, ev,
+                                   0, (const DevObject *)nullptr, (const DevParams *)nullptr);
+}
+
 int launch_eval(const DevObject &o, const DevParams &p, EvalOut ev, double *scratch, void *stream)
 {
+    TeamLaunch l;
+    for (int k = 2; k >= 0; --k) {
+        if (max_teams(o, kTeamSizes[k]) < 1) continue;
+        const int e = l.prepare(o, 1, kTeamSizes[k], stream);
+        if (e) return e;
+        return (int)cudaLaunchKernelEx(&l.cfg, l.fn, o, p, (const FitItem *)nullptr, 1, (int *)nullptr,
+                                       (FitOut *)nullptr, scratch, (size_t)0, (int *)nullptr, ev, 1,
+                                       (const DevObject *)nullptr, (const DevParams *)nullptr);
+    }
     KernelFn fn;
     size_t smem;
-    int e = prepare_kernel(o, &fn, &smem);
+    const int e = prepare_kernel(o, &fn, &smem);
     if (e) return e;
     fn<<<1, kThreads, smem, (cudaStream_t)stream>>>(o, p, nullptr, 1, nullptr, nullptr, scratch, 0, nullptr,
                                                     ev, 1, nullptr, nullptr);

@@ -24,6 +24,7 @@ struct DevObject {
     int cstat_smem;           // 1: per-curve statistics live in shared memory (they fit)
     const double4 *facet;     // [n_fac] {nx, ny, nz, d_area}
     const double *ysh;        // [n_fac][ncp] Laplace basis, zero-padded to ncp
+    const double *ysh_t;      // [n_coef][n_fac] the same transposed, or nullptr (no room)
     const double4 *pt_a;      // [n_points] {t, ee.x, ee.y, ee.z}
     const double4 *pt_b;      // [n_points] {ee0.x, ee0.y, ee0.z, brightness}
     const double *pt_w;       // [n_points] sigr2 * weight
@@ -94,11 +95,26 @@ int padded_ncoef(int n_coef);
 int launch_fits(const DevObject &o, const DevParams &p, const FitItem *items, int n_items,
                 int *queue, FitOut *out, double *scratch, size_t scratch_per_cta, int n_ctas,
                 int *status, void *stream);
-// One evaluation at ev.a, 1 CTA.  rows_out (optional): [n_points][row_stride].
+// One evaluation at ev.a by a team of CTAs on one scratch slab.
 int launch_eval(const DevObject &o, const DevParams &p, EvalOut ev, double *scratch,
                 void *stream);
 // CTAs per SM the fit kernel reaches for this object.
 int fit_ctas_per_sm(const DevObject &o);
+
+// How n fits of one object are spread over the GPU: the first main_items by
+// single CTAs, the rest by teams (clusters of team_size CTAs per fit).
+struct FitPlan {
+    int main_items = 0, main_ctas = 0;
+    int team_items = 0, teams = 0, team_size = 1;
+    int slabs() const { return main_ctas + teams; }  // scratch slabs in use at a time
+};
+// resident: CTAs the GPU holds; max_slabs: scratch slabs there is room for (0:
+// any number); mixable: the two kinds may run side by side (two streams).
+FitPlan plan_fits(const DevObject &o, int n, int resident, int max_slabs, bool mixable);
+// Launches one kind of a plan: team_size CTAs per fit, `groups` fits at a time.
+int launch_fit_teams(const DevObject &o, const DevParams &p, const FitItem *items, int n_items, int *queue,
+                     FitOut *out, double *scratch, size_t scratch_per_cta, int groups, int team_size, int *status,
+                     void *stream);
 
 // Many objects of one padded coefficient count in one persistent launch (FP64
 // kernel).  env carries the largest sizes of the objects (the shared-memory

@@ -154,6 +154,47 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, uint32_t pari
     return false;
 }
 
+// The CTAs that work on one fit: one, or a thread-block cluster of 2, 4 or 8
+// that shares the fit's scratch slab in global memory.  Every CTA of a cluster
+// holds the fit's whole state and takes the same decisions; the points of the
+// sweeps, the curves and the blocks of the normal matrix are dealt out.  What
+// one CTA writes to the slab and another reads goes through L2 (load()) after
+// a sync().
+template <bool CL>
+struct Team {
+    __device__ __forceinline__ int rank() const
+    {
+        if constexpr (!CL) return 0;
+        uint32_t r;
+        asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+        return (int)r;
+    }
+    __device__ __forceinline__ int size() const
+    {
+        if constexpr (!CL) return 1;
+        uint32_t r;
+        asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+        return (int)r;
+    }
+    // the scratch slab, work item and result of this CTA's fit
+    __device__ __forceinline__ int index() const { return CL ? blockIdx.x / size() : blockIdx.x; }
+    __device__ __forceinline__ void sync() const
+    {
+        if constexpr (CL) {
+            asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+        } else {
+            __syncthreads();
+        }
+    }
+    template <typename T>
+    __device__ __forceinline__ T load(const T *p) const
+    {
+        if constexpr (CL) return __ldcg(p);
+        return *p;
+    }
+};
+
 // Charges the cycles since the previous mark to `phase` (thread 0, when the
 // caller asked for phase clocks).
 __device__ __forceinline__ void tmark(const DevParams &p, const Sh &s, int phase)
@@ -302,14 +343,29 @@ __device__ __forceinline__ void block_sum(double *v, double *red)
 static __device__ double shape_areas(const DevObject &o, const Sh &s, const double *a)
 {
     double part = 0;
-    const int nc = o.n_coef;
-    for (int f = threadIdx.x; f < o.n_fac; f += kThreads) {
-        const double *y = o.ysh + (size_t)f * o.ncp;
-        double g = 0;
-        for (int k = 0; k < nc; ++k) g += a[k + 1] * __ldg(y + k);
-        double ar = __ldg(&o.facet[f].w) * exp(g);
+    const int nc = o.n_coef, nf = o.n_fac;
+    for (int f = threadIdx.x; f < nf; f += 2 * kThreads) {
+        // thread = facet, two at a time: from the transposed basis a warp's
+        // loads are coalesced (49 coefficients, 512 facets: with the invariants
+        // 23e3 -> 6e3 cycles)
+        const int f2 = f + kThreads < nf ? f + kThreads : f;
+        const double *y = o.ysh_t ? o.ysh_t + f : o.ysh + (size_t)f * o.ncp;
+        const double *y2 = o.ysh_t ? o.ysh_t + f2 : o.ysh + (size_t)f2 * o.ncp;
+        const size_t ks = o.ysh_t ? nf : 1;
+        double g = 0, g2 = 0;
+#pragma unroll 8
+        for (int k = 0; k < nc; ++k) {
+            g += a[k + 1] * __ldg(y + k * ks);
+            g2 += a[k + 1] * __ldg(y2 + k * ks);
+        }
+        const double ar = __ldg(&o.facet[f].w) * exp(g);
         s.F[f].w = ar;
         part += ar;
+        if (f2 != f) {
+            const double ar2 = __ldg(&o.facet[f2].w) * exp(g2);
+            s.F[f2].w = ar2;
+            part += ar2;
+        }
     }
     double v[1] = {part};
     block_sum<1>(v, s.red);
@@ -460,15 +516,30 @@ __device__ __forceinline__ void point_geometry(const double *inv, double t, cons
 // nearly the same facets and whole warps skip facets none of them sees.  Rows
 // are written at the original point index and every skipped term is an exact
 // zero, so the order changes nothing in the results.
-static __device__ void sort_points(const DevObject &o, const Sh &s, int *perm, int *keys)
+// A team's CTAs each take a contiguous share of the points: the share's counts
+// per cell go to `counts` ([team][cells], global), and every CTA adds them up
+// to where its own points of each cell start.
+template <bool CL>
+static __device__ void sort_points(const DevObject &o, const Sh &s, int *perm, int *keys, int *counts)
 {
+    const Team<CL> team;
     const int tid = threadIdx.x, np = o.n_points;
+    const int share = (np + team.size() - 1) / team.size();
+    const int q0 = team.rank() * share, q1 = min(np, q0 + share);
     int *hist = s.hist, *offs = s.hist + kSortCells;
     for (int c = tid; c < kSortCells; c += kThreads) hist[c] = 0;
     __syncthreads();
-    for (int q = tid; q < np; q += kThreads) {
-        const double4 pa = ldg4(&o.pt_a[q]);
-        const double4 pb = ldg4(&o.pt_b[q]);
+    double4 na, nb;  // the next point, read one ahead
+    if (q0 + tid < q1) {
+        na = ldg4(&o.pt_a[q0 + tid]);
+        nb = ldg4(&o.pt_b[q0 + tid]);
+    }
+    for (int q = q0 + tid; q < q1; q += kThreads) {
+        const double4 pa = na, pb = nb;
+        if (q + kThreads < q1) {
+            na = ldg4(&o.pt_a[q + kThreads]);
+            nb = ldg4(&o.pt_b[q + kThreads]);
+        }
         const double ee[3] = {pa.y, pa.z, pa.w}, es[3] = {pb.x, pb.y, pb.z};
         PointGeo g;
         point_geometry<kGeoDirections>(s.inv, pa.x, ee, es, g);
@@ -489,6 +560,22 @@ static __device__ void sort_points(const DevObject &o, const Sh &s, int *perm, i
         atomicAdd(&hist[key], 1);
     }
     __syncthreads();
+    if constexpr (CL) {
+        team.sync();  // the partial sums that lay there have been read
+        for (int c = tid; c < kSortCells; c += kThreads) counts[team.rank() * kSortCells + c] = hist[c];
+        team.sync();
+        for (int c = tid; c < kSortCells; c += kThreads) {
+            int before = 0, all = 0;
+            for (int r = 0; r < team.size(); ++r) {
+                const int n = team.load(&counts[r * kSortCells + c]);
+                if (r < team.rank()) before += n;
+                all += n;
+            }
+            hist[c] = all;
+            offs[c] = before;
+        }
+        __syncthreads();
+    }
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x, per = kSortCells / 32;
         int local[kSortCells / 32], sum = 0;
@@ -506,13 +593,13 @@ static __device__ void sort_points(const DevObject &o, const Sh &s, int *perm, i
         int run = incl - sum;
 #pragma unroll
         for (int i = 0; i < per; ++i) {
-            offs[lane * per + i] = run;
+            offs[lane * per + i] = CL ? offs[lane * per + i] + run : run;
             run += local[i];
         }
     }
     __syncthreads();
-    for (int q = tid; q < np; q += kThreads) perm[atomicAdd(&offs[keys[q]], 1)] = q;
-    __syncthreads();
+    for (int q = q0 + tid; q < q1; q += kThreads) perm[atomicAdd(&offs[keys[q]], 1)] = q;
+    team.sync();
 }
 
 // Brightness and raw derivative rows of all points: mrqcof_curve1_opt
@@ -583,7 +670,7 @@ __device__ __forceinline__ unsigned group_mask(const float4 *cone, int nfc, bool
 // step) and the block's MMAs are skipped: they would spend 8 columns of tensor
 // work on one.  The lane's accumulator is element C[0][NT - 1][0], which the
 // skipped MMAs leave free.
-template <int NCP, bool X1>
+template <int NCP, bool X1, bool CL>
 __device__ void brightness_rows(const DevObject &o, const Sh &s, double *rows, const int *perm)
 {
     constexpr int NT = NCP / 8;
@@ -594,7 +681,8 @@ __device__ void brightness_rows(const DevObject &o, const Sh &s, double *rows, c
     const int fc = chunk_facets(NCP);
     const int nchunks = (nf + fc - 1) / fc;
     const int ntiles = (np + 31) / 32;
-    const int nrounds = (ntiles + kWarps - 1) / kWarps;
+    const Team<CL> team;
+    const int nrounds = (ntiles + kWarps * team.size() - 1) / (kWarps * team.size());
     const int total = nrounds * nchunks;
     double *wt = s.wst + warp * 32 * 4;
     bool timeout = false;
@@ -611,11 +699,13 @@ __device__ void brightness_rows(const DevObject &o, const Sh &s, double *rows, c
 
     int g = 0;
     for (int round = 0; round < nrounds; ++round) {
-        const int tile = round * kWarps + warp;
+        // a CTA's tiles of a round are neighbours: they see the same facets, so
+        // its warps keep pace over the basis chunks
+        const int tile = (round * team.size() + team.rank()) * kWarps + warp;
         const bool tile_act = tile < ntiles;
         const int idx = tile * 32 + lane;
         const bool act = tile_act && idx < np;
-        const int p = perm[min(idx, np - 1)];
+        const int p = team.load(&perm[min(idx, np - 1)]);
         double ex, ey, ez, sx, sy, sz;
         {
             const double4 pa = ldg4(&o.pt_a[p]);
@@ -866,7 +956,7 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], 
 // floats, zero-padded past the last facet.  One warp = 32 points, steps of 8
 // facets (the MMA's k); a step no lane sees is skipped whole, a 16-point half
 // that sees none of its 8 facets skips its MMAs.
-template <int NCP>
+template <int NCP, bool CL>
 __device__ void brightness_rows_mixed(const DevObject &o, const Sh &s, double *rows, const int *perm)
 {
     constexpr int NT = NCP / 8;
@@ -877,7 +967,8 @@ __device__ void brightness_rows_mixed(const DevObject &o, const Sh &s, double *r
     const int fc = chunk_facets(NCP);
     const int nchunks = (nf + fc - 1) / fc;
     const int ntiles = (np + 31) / 32;
-    const int nrounds = (ntiles + kWarps - 1) / kWarps;
+    const Team<CL> team;
+    const int nrounds = (ntiles + kWarps * team.size() - 1) / (kWarps * team.size());
     const int total = nrounds * nchunks;
     float *whi = s.wst32 + warp * 2 * 32 * kWS;
     float *wlo = whi + 32 * kWS;
@@ -895,11 +986,13 @@ __device__ void brightness_rows_mixed(const DevObject &o, const Sh &s, double *r
 
     int gi = 0;
     for (int round = 0; round < nrounds; ++round) {
-        const int tile = round * kWarps + warp;
+        // a CTA's tiles of a round are neighbours: they see the same facets, so
+        // its warps keep pace over the basis chunks
+        const int tile = (round * team.size() + team.rank()) * kWarps + warp;
         const bool tile_act = tile < ntiles;
         const int idx = tile * 32 + lane;
         const bool act = tile_act && idx < np;
-        const int p = perm[min(idx, np - 1)];
+        const int p = team.load(&perm[min(idx, np - 1)]);
         float ex, ey, ez, sx, sy, sz;
         {
             const double4 pa = ldg4(&o.pt_a[p]);
@@ -1203,6 +1296,41 @@ __device__ __forceinline__ void syrk_add_block(const Sh &s, int mfit, int bj, in
     }
 }
 
+// Adds the partial sums (kWarps, or a single one) of the lower blocks, in order,
+// into alpha (both triangles), beta and chi^2.
+template <bool CL>
+__device__ __forceinline__ void syrk_reduce(const Sh &s, int mfit, int nblocks, int parts, double *dst, double *dvec,
+                                            const double *gpart)
+{
+    const Team<CL> team;
+    const int ld = s.ld, stride = parts > 1 ? kSliceBlk * 64 : 0;
+    for (int idx = threadIdx.x; idx < nblocks * 64; idx += kThreads) {
+        const int i = idx >> 6, l = (idx >> 1) & 31, e = idx & 1;
+        double v = 0.0;
+        if (parts > 1) {
+            double t[kWarps];  // all in flight, added in order
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) t[w] = team.load(&gpart[(size_t)w * stride + (i * 32 + l) * 2 + e]);
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) v += t[w];
+        } else {
+            v += team.load(&gpart[(i * 32 + l) * 2 + e]);
+        }
+        int bj = 0;
+        while ((bj + 1) * (bj + 2) / 2 <= i) ++bj;
+        const int bk = i - bj * (bj + 1) / 2;
+        const int row = 8 * bj + (l >> 2), col = 8 * bk + 2 * (l & 3) + e;
+        if (row < mfit && col <= row) {
+            dst[row * ld + col] = v;
+            dst[col * ld + row] = v;
+        } else if (row == mfit && col < mfit) {
+            dvec[col] = v;
+        } else if (row == mfit && col == mfit) {
+            s.scal[S_TRIAL] = v;
+        }
+    }
+}
+
 // Writes the accumulated alpha, beta and chi^2 (all threads call this).  In
 // k-slice mode the 8 warps' partial sums go through a scratch slab (L2) and
 // are added in warp order, element by element, by all threads.
@@ -1217,24 +1345,7 @@ __device__ __forceinline__ void syrk_store(const Sh &s, int mfit, const SyrkAcc 
         for (int i = 0; i < kSliceBlk; ++i)
             if (i < nblocks) mine[i * 32 + lane] = make_double2(acc.c[i][0], acc.c[i][1]);
         __syncthreads();
-        const int ld = s.ld;
-        for (int idx = tid; idx < nblocks * 64; idx += kThreads) {
-            const int i = idx >> 6, l = (idx >> 1) & 31, e = idx & 1;
-            double v = 0.0;
-            for (int w = 0; w < kWarps; ++w) v += gpart[((size_t)w * kSliceBlk * 32 + i * 32 + l) * 2 + e];
-            int bj = 0;
-            while ((bj + 1) * (bj + 2) / 2 <= i) ++bj;
-            const int bk = i - bj * (bj + 1) / 2;
-            const int row = 8 * bj + (l >> 2), col = 8 * bk + 2 * (l & 3) + e;
-            if (row < mfit && col <= row) {
-                dst[row * ld + col] = v;
-                dst[col * ld + row] = v;
-            } else if (row == mfit && col < mfit) {
-                dvec[col] = v;
-            } else if (row == mfit && col == mfit) {
-                s.scal[S_TRIAL] = v;
-            }
-        }
+        syrk_reduce<false>(s, mfit, nblocks, kWarps, dst, dvec, gpart);
         __syncthreads();
         return;
     }
@@ -1257,11 +1368,245 @@ static __device__ void moment_sums(const DevObject &o, const Sh &s, double (&r)[
     block_sum<3>(r, s.red);
 }
 
+// Raw derivatives d ym_i / d a_k of the pseudo-points for shape coefficient
+// k = tid: groups of nc threads take consecutive facet ranges, their partial
+// sums (staged in the idle tile buffer) are added in group order.
+static __device__ void pseudo_derivatives(const DevObject &o, const Sh &s, double (&dk)[3])
+{
+    const int tid = threadIdx.x, nc = o.n_coef, nf = o.n_fac;
+    const int ngrp = max(1, min(kThreads / nc, (s.tr * s.mfp) / (3 * nc)));
+    const int per = (nf + ngrp - 1) / ngrp;
+    const int grp = tid / nc, k = tid - grp * nc;
+    if (grp < ngrp) {
+        double pk[3] = {0, 0, 0};
+        const int fe = min(nf, (grp + 1) * per);
+        auto add = [&](int fi, double y) {
+            const double4 fr = s.F[fi];
+            pk[0] += (fr.w * fr.x) * y;
+            pk[1] += (fr.w * fr.y) * y;
+            pk[2] += (fr.w * fr.z) * y;
+        };
+        constexpr int kAhead = 16;  // basis loads in flight
+        const double *yk = o.ysh + k;
+        int fi = grp * per;
+        for (; fi + kAhead <= fe; fi += kAhead) {
+            double y[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) y[u] = __ldg(yk + (size_t)(fi + u) * o.ncp);
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) add(fi + u, y[u]);
+        }
+        for (; fi < fe; ++fi) add(fi, __ldg(yk + (size_t)fi * o.ncp));
+#pragma unroll
+        for (int i = 0; i < 3; ++i) s.T[(grp * 3 + i) * nc + k] = pk[i];
+    }
+    __syncthreads();
+    dk[0] = dk[1] = dk[2] = 0;
+    if (tid < nc)
+        for (int g = 0; g < ngrp; ++g)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) dk[i] += s.T[(g * 3 + i) * nc + tid];
+    __syncthreads();
+}
+
+// The three pseudo-points as rows 0..2 of the staged tile, zeros below.
+static __device__ void stage_pseudo_rows(const DevObject &o, const Sh &s, const double (&ym)[3], const double (&dk)[3],
+                                         double conw_r)
+{
+    const int tid = threadIdx.x, nc = o.n_coef, mfit = o.mfit, mfp = s.mfp;
+    const double wps = conw_r * conw_r;
+    for (int idx = tid; idx < kTile * mfp; idx += kThreads) {
+        s.T[idx] = 0.0;
+        s.TW[idx] = 0.0;
+    }
+    __syncthreads();
+    if (tid < nc) {
+        int slot = -1;  // fit slot of parameter tid + 1, if fitted
+        for (int j = 0; j < mfit; ++j)
+            if (s.fidx[j] == tid + 1) slot = j;
+        if (slot >= 0)
+            for (int i = 0; i < 3; ++i) {
+                s.T[i * mfp + slot] = dk[i];
+                s.TW[i * mfp + slot] = dk[i] * wps;
+            }
+    }
+    if (tid < 3) {
+        const double dy = 0.0 - ym[tid];
+        s.T[tid * mfp + mfit] = dy;
+        s.TW[tid * mfp + mfit] = dy * wps;
+    }
+}
+
+// J^T W J, J^T W dy and chi^2 by a team: the same k-steps in the same order
+// for every element as one CTA's update, so the bits agree.  k-slice mode: the
+// 8 row slices are dealt to the CTAs and a slice's blocks to the warps of its
+// CTA; block mode: the blocks are dealt to all warps of the team and every CTA
+// stages all rows.  A batch of tile_rows rows is staged at a time (row loads
+// of the next batch in flight under the MMAs), 4 rows a k-step.
+//
+template <int TS>
+static __device__ __noinline__ void normal_matrix_team(const DevObject &o, const Sh &s, const double *rows,
+                                                       const double *cstat, double *dst, double *dvec, double *gpart,
+                                                       double conw_r)
+{
+    const Team<true> team;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int np = o.n_points, ma = o.ma, mfit = o.mfit, mfp = s.mfp, RS = o.row_stride, CS = ma + 3;
+    const int nb = fit_mpad(mfit) / 8, nblocks = nb * (nb + 1) / 2;
+    const bool slice = syrk_slices(mfit, s.tr);
+    constexpr int per_cta = kWarps / TS;                 // k-slice mode: slices of this CTA
+    const int mine = warp / TS;                          // ... the one of this warp
+    const int part = slice ? warp % TS : team.rank() * kWarps + warp;
+    const int nparts = slice ? TS : kWarps * TS;
+    constexpr int kBlk = (kSliceBlk + TS - 1) / TS;      // blocks of one warp, at most
+    static_assert(kBlk >= (78 + kWarps * TS - 1) / (kWarps * TS), "block mode has fewer");
+    double c[kBlk][2];
+    int oa[kBlk], ob[kBlk], nblk = 0;
+#pragma unroll
+    for (int j = 0; j < kBlk; ++j) {
+        const int i = part + j * nparts;
+        int bj = 0;
+        while ((bj + 1) * (bj + 2) / 2 <= i) ++bj;
+        // accumulators past the last block run on block (0, 0) and are dropped
+        oa[j] = i < nblocks ? 8 * bj : 0;
+        ob[j] = i < nblocks ? 8 * (i - bj * (bj + 1) / 2) : 0;
+        if (i < nblocks) nblk = j + 1;
+        c[j][0] = c[j][1] = 0.0;
+    }
+    const int TR = s.tr, nks = TR / 4, rpw = TR / kWarps;  // k-steps a batch, rows a warp stages
+    const int ntile = (np + kTile - 1) / kTile;
+    const int nbatch = slice ? (ntile + TS - 1) / TS : (np + TR - 1) / TR;
+    // point of staged row r of batch b
+    auto point = [&](int b, int r) {
+        if (!slice) return b * TR + r;
+        const int ks = r >> 2;
+        return (b * TS + ks / per_cta) * kTile + 4 * (team.rank() * per_cta + ks % per_cta) + (r & 3);
+    };
+    constexpr int kChunks = 3;  // columns lane, lane + 32, lane + 64 (mfit + 1 <= 90)
+    int col[kChunks];           // raw-row column of this lane's fit columns
+#pragma unroll
+    for (int u = 0; u < kChunks; ++u) col[u] = s.fidx[min(lane + 32 * u, mfit - 1)] - 1;
+    const int kq = lane & 3, cq = lane >> 2;
+    constexpr int kBlockMode = (78 + kWarps * TS - 1) / (kWarps * TS);
+    auto step = [&](auto blocks, int ks) {
+        constexpr int N = decltype(blocks)::value;
+        const double *tw = s.TW + (4 * ks + kq) * mfp + cq, *tt = s.T + (4 * ks + kq) * mfp + cq;
+        constexpr int kHold = 6;  // operands held at a time
+#pragma unroll
+        for (int j0 = 0; j0 < N; j0 += kHold) {
+            double fa[kHold], fb[kHold];
+#pragma unroll
+            for (int j = 0; j < kHold; ++j)
+                if (j0 + j < N) {
+                    fa[j] = tw[oa[j0 + j]];
+                    fb[j] = tt[ob[j0 + j]];
+                }
+#pragma unroll
+            for (int j = 0; j < kHold; ++j)
+                if (j0 + j < N) dmma_8x8x4(c[j0 + j][0], c[j0 + j][1], fa[j], fb[j]);
+        }
+    };
+    auto steps = [&](int n) {
+        if (slice) {
+#pragma unroll 2
+            for (int ks = mine; ks < n; ks += per_cta) step(std::integral_constant<int, kBlk>{}, ks);
+        } else {
+#pragma unroll 2
+            for (int ks = 0; ks < n; ++ks) step(std::integral_constant<int, kBlockMode>{}, ks);
+        }
+    };
+    // The rows of the next batch are in flight under this one's MMAs.  (Two or
+    // four batches ahead were slower: the longer code costs every phase of the
+    // kernel instruction-cache misses.)
+    auto run = [&](auto rows_per_warp) {
+        constexpr int RP = decltype(rows_per_warp)::value;
+        double raw[RP][kChunks];
+        double4 rec = make_double4(0, 0, 0, 0);  // lane k < RP: the record and brightness of staged row k
+        double ym0 = 0;
+        auto fetch = [&](int b) {
+            if (lane < RP) {
+                const int q = min(point(b, warp * RP + lane), np - 1);
+                rec = ldg4(&o.pt_rec[q]);
+                ym0 = team.load(&rows[(size_t)q * RS + ma]);
+            }
+#pragma unroll
+            for (int k = 0; k < RP; ++k) {
+                const double *row = rows + (size_t)min(point(b, warp * RP + k), np - 1) * RS;
+#pragma unroll
+                for (int u = 0; u < kChunks; ++u)
+                    if (32 * u < mfit) raw[k][u] = team.load(&row[col[u]]);
+            }
+        };
+        fetch(0);
+        for (int b = 0; b < nbatch; ++b) {
+            // per-row scalars: lane k < RP computes row warp * RP + k
+            const bool okL = lane < RP && point(b, warp * RP + lane) < np;
+            const bool relL = okL && rec.w != 0.0;
+            const int curL = relL ? (int)rec.z : -1;
+            const double coefL = relL ? s.ccoef[max(curL, 0)] : 0.0;
+            const double subL = relL ? ym0 * s.crave[max(curL, 0)] : 0.0;
+            const double ymodL = relL ? coefL * ym0 : ym0;
+            const double dyL = okL ? rec.x - ymodL : 0.0;
+            const double wL = okL ? rec.y : 0.0;
+#pragma unroll
+            for (int k = 0; k < RP; ++k) {
+                const bool valid = point(b, warp * RP + k) < np;
+                const double dy = __shfl_sync(0xffffffffu, dyL, k);
+                const double w = __shfl_sync(0xffffffffu, wL, k);
+                const double coef = __shfl_sync(0xffffffffu, coefL, k);
+                const double sub = __shfl_sync(0xffffffffu, subL, k);
+                const int cur = __shfl_sync(0xffffffffu, curL, k);
+                const bool rel = cur >= 0;
+                const double *dav = cstat + (size_t)max(cur, 0) * CS;  // neighbouring rows: the same curve, L1 hits
+                double *trow = s.T + (warp * RP + k) * mfp, *twrow = s.TW + (warp * RP + k) * mfp;
+#pragma unroll
+                for (int u = 0; u < kChunks; ++u) {
+                    const int j = lane + 32 * u;
+                    if (j < mfp) {
+                        const double dv = rel ? dav[col[u]] : 0.0;
+                        double v = rel ? coef * (raw[k][u] - sub * dv) : raw[k][u];
+                        v = j < mfit ? v : (j == mfit ? dy : 0.0);
+                        v = valid ? v : 0.0;
+                        trow[j] = v;
+                        twrow[j] = v * w;
+                    }
+                }
+            }
+            __syncthreads();
+            if (b + 1 < nbatch) fetch(b + 1);
+            steps(nks);
+            __syncthreads();
+        }
+    };
+    if (rpw == 4)
+        run(std::integral_constant<int, 4>{});
+    else
+        run(std::integral_constant<int, 2>{});
+    // convexity regularisation pseudo-points: one more k-step of slice 0
+    if (!slice || team.rank() == 0) {
+        double ym[3], dk[3];
+        moment_sums(o, s, ym);
+        pseudo_derivatives(o, s, dk);
+        stage_pseudo_rows(o, s, ym, dk, conw_r);
+        __syncthreads();
+        if (!slice || mine == 0) steps(1);
+    }
+    const int at = slice ? (team.rank() * per_cta + mine) * kSliceBlk : 0;
+#pragma unroll
+    for (int j = 0; j < kBlk; ++j)
+        if (j < nblk)
+            reinterpret_cast<double2 *>(gpart)[(at + part + j * nparts) * 32 + lane] = make_double2(c[j][0], c[j][1]);
+    team.sync();
+    syrk_reduce<true>(s, mfit, nblocks, slice ? kWarps : 1, dst, dvec, gpart);
+    __syncthreads();
+}
+
 // What an evaluation at parameter vector a starts with: facet areas, their
 // sum (S_AREA), the invariants, in mixed precision the FP32 facet tables, and
 // the point order.
-template <bool MIXED>
-static __device__ void evaluation_setup(const DevObject &o, const DevParams &p, const Sh &s, const double *a, int *perm)
+template <bool MIXED, bool CL>
+static __device__ void evaluation_setup(const DevObject &o, const DevParams &p, const Sh &s, const double *a,
+                                        double *rows, int *perm)
 {
     const int tid = threadIdx.x;
     if (tid == 0) s.ctl[C_NEXT] = 0;
@@ -1278,16 +1623,18 @@ static __device__ void evaluation_setup(const DevObject &o, const DevParams &p, 
         __syncthreads();
     }
     tmark(p, s, T_CURV);
-    sort_points(o, s, perm, perm + o.n_points);
+    // the counts' place: the partial sums of the rank-k update, idle now
+    sort_points<CL>(o, s, perm, perm + o.n_points,
+                    reinterpret_cast<int *>(rows + scratch_gpart(o.n_points, o.row_stride, o.n_curves, o.ma)));
     tmark(p, s, T_SORT);
 }
 
 // 1 / sum(ymod) and the renormalisation coefficient of relative curve c.
-__device__ __forceinline__ void renormalise_curve(const DevObject &o, const Sh &s, int c, double sum)
+__device__ __forceinline__ void renormalise_curve(const Sh &s, int c, double sum, double sigma, int points)
 {
     const double rave = 1.0 / sum;
     s.crave[c] = rave;
-    s.ccoef[c] = o.curve_sig[c] * (o.curve_start[c + 1] - o.curve_start[c]) * rave;
+    s.ccoef[c] = sigma * points * rave;
 }
 
 // ---------------------------------------------------------------- trial steps
@@ -1302,20 +1649,21 @@ __device__ __forceinline__ void renormalise_curve(const DevObject &o, const Sh &
 // per lane, their stages written side by side.  Visibility by integer
 // comparison of the bit patterns, which spares the FP64 pipe two operations a
 // facet, was 6 % slower: the integer instructions cost more issue slots.
-template <bool MIXED>
+template <bool MIXED, bool CL>
 static __device__ void brightness_only(const DevObject &o, const Sh &s, double *ym, const int *perm)
 {
+    const Team<CL> team;
     const int lane = threadIdx.x & 31;
     const int np = o.n_points, nf = o.n_fac, ntiles = (np + 31) / 32;
     const double cl = s.inv[5], cls = s.inv[6];
     for (;;) {
         int tile = 0;
         if (lane == 0) tile = atomicAdd(&s.ctl[C_NEXT], 1);
-        tile = __shfl_sync(0xffffffffu, tile, 0);
+        tile = __shfl_sync(0xffffffffu, tile, 0) * team.size() + team.rank();
         if (tile >= ntiles) break;
         const int idx = tile * 32 + lane;
         const bool act = idx < np;
-        const int p = perm[min(idx, np - 1)];
+        const int p = team.load(&perm[min(idx, np - 1)]);
         PointGeo geo;
         {
             const double4 pa = ldg4(&o.pt_a[p]);
@@ -1436,85 +1784,149 @@ static __device__ void brightness_only(const DevObject &o, const Sh &s, double *
 // (perm) of the trial parameters for the full evaluation that follows an
 // accepted step, the summed area in S_AREA and the summed area-weighted
 // normals in S_MOM.  All threads must call it.
-template <bool MIXED>
+template <bool MIXED, bool CL>
 static __device__ double trial_chisq(const DevObject &o, const DevParams &p, const Sh &s, double *rows, int *perm,
                                      double conw_r)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const Team<CL> team;
     const int np = o.n_points, mfit = o.mfit;
     tmark(p, s, T_REST);
-    evaluation_setup<MIXED>(o, p, s, s.atry, perm);
+    evaluation_setup<MIXED, CL>(o, p, s, s.atry, rows, perm);
 
-    // per point: model brightness, then residual and weighted residual -- in
-    // the idle tile storage if they fit there, else in the row slab
-    double *dy = 2 * sizeof(double) * (size_t)np <= s.un_bytes ? s.ybuf : rows;
-    double *dyw = dy + np;
-    brightness_only<MIXED>(o, s, dy, perm);
-    __syncthreads();
+    int cp0 = 0, cp1 = 0, crel = 0;  // this thread's first curve
+    double csig = 0;
+    if (tid < o.n_curves) {
+        cp0 = __ldg(&o.curve_start[tid]);
+        cp1 = __ldg(&o.curve_start[tid + 1]);
+        crel = __ldg(&o.curve_rel[tid]);
+        csig = __ldg(&o.curve_sig[tid]);
+    }
+    // model brightness of all points: in the idle tile storage if it fits there
+    // beside the residual chunks below, else in the row slab
+    const size_t kLeast = 4 * 256 * sizeof(double);
+    const bool local = sizeof(double) * (size_t)np + kLeast <= s.un_bytes;
+    double *y = local ? s.ybuf : rows;
+    if constexpr (CL) {
+        // every CTA sweeps its tiles into the slab and then goes on with all points
+        brightness_only<MIXED, CL>(o, s, rows, perm);
+        team.sync();
+        if (local) {
+            constexpr int kAhead = 8;
+            for (int qb = tid; qb < np; qb += kAhead * kThreads) {
+                double v[kAhead];
+#pragma unroll
+                for (int u = 0; u < kAhead; ++u) v[u] = team.load(&rows[min(qb + u * kThreads, np - 1)]);
+#pragma unroll
+                for (int u = 0; u < kAhead; ++u)
+                    if (qb + u * kThreads < np) y[qb + u * kThreads] = v[u];
+            }
+            __syncthreads();
+        }
+    } else {
+        brightness_only<MIXED, CL>(o, s, y, perm);
+        __syncthreads();
+    }
     tmark(p, s, T_TRIAL);
+    auto get = [&](const double *v) { return CL && !local ? team.load(v) : *v; };
     // renormalisation of the relative curves: one thread per curve adds its
     // points in order
     for (int c = tid; c < o.n_curves; c += kThreads) {
-        if (!o.curve_rel[c]) continue;
-        const int p0 = o.curve_start[c], p1 = o.curve_start[c + 1];
+        const bool own = c == tid;  // read ahead of the sweep
+        const int p0 = own ? cp0 : o.curve_start[c], p1 = own ? cp1 : o.curve_start[c + 1];
+        const double cs = own ? csig : o.curve_sig[c];
+        if (!(own ? crel : o.curve_rel[c])) continue;
         double sum = 0;
-        constexpr int kAhead = 8;
-        for (int q0 = p0; q0 < p1; q0 += kAhead) {
+        constexpr int kAhead = 16;
+        int q = p0;
+        for (; q + kAhead <= p1; q += kAhead) {
             double v[kAhead];
 #pragma unroll
-            for (int u = 0; u < kAhead; ++u) v[u] = q0 + u < p1 ? dy[q0 + u] : 0.0;
+            for (int u = 0; u < kAhead; ++u) v[u] = get(&y[q + u]);
 #pragma unroll
             for (int u = 0; u < kAhead; ++u) sum += v[u];
         }
-        renormalise_curve(o, s, c, sum);
+        for (; q < p1; ++q) sum += get(&y[q]);
+        renormalise_curve(s, c, sum, cs, p1 - p0);
     }
     // area-weighted normals: the pseudo-points' residuals
     double ym[3];
     moment_sums(o, s, ym);  // its barriers also order the coefficients above
     if (tid == 0)
         for (int i = 0; i < 3; ++i) s.scal[S_MOM + i] = ym[i];
-    for (int q = tid; q < np; q += kThreads) {
-        const double4 rec = ldg4(&o.pt_rec[q]);
-        double ymod = dy[q];
-        if (rec.w != 0.0) ymod = __dmul_rn(s.ccoef[(int)rec.z], ymod);
-        const double d = __dsub_rn(rec.x, ymod);
-        dy[q] = d;
-        dyw[q] = __dmul_rn(d, rec.y);
-    }
-    __syncthreads();
 
     // chi^2 as the full evaluation's tensor-core update forms it: element
     // (mfit, mfit) of the augmented matrix, the same MMA steps in the same
     // order with every other column zero.  k-slice mode: warp w adds rows
     // 4w..4w+3 of every 32; block mode: the warp that owns the last block
-    // adds 4 rows a step.  The pseudo-points come last.
+    // adds 4 rows a step.  The pseudo-points come last.  The residuals and
+    // weighted residuals of the next chunk of points are formed while the
+    // chains of MMAs run over this one's.
     const int nb = fit_mpad(mfit) / 8;
     const bool slice = syrk_slices(mfit, s.tr);
     const int owner = slice ? 0 : (nb * (nb + 1) / 2 - 1) & (kWarps - 1);
     const int m = mfit & 7, k = lane & 3;
     const bool col = (lane >> 2) == m;
-    double c0 = 0.0, c1 = 0.0;
-    if (slice || warp == owner) {
-        const int step = slice ? 4 * kWarps : 4;
-        constexpr int kAhead = 8;
-        for (int q0 = (slice ? 4 * warp : 0); q0 < ((np + step - 1) / step) * step; q0 += kAhead * step) {
-            double fa[kAhead], fb[kAhead];
+    double *buf = s.ybuf + (local ? np + (np & 1) : 0);
+    const int room = (int)((s.un_bytes / sizeof(double) - (buf - s.ybuf)) / 4);
+    const int chunk = min(room & ~31, (np + 31) & ~31), nchunk = (np + chunk - 1) / chunk;
+    // in block mode the owner's warp leaves the staging to the others
+    const bool stager = slice || warp != owner;
+    const int st0 = slice || warp < owner ? tid : tid - 32, stn = slice ? kThreads : kThreads - 32;
+    auto stage = [&](int c) {
+        double *dy = buf + (c & 1) * 2 * chunk, *dyw = dy + chunk;
+        const int q0 = c * chunk, q1 = min(np, q0 + chunk);
+        constexpr int kAhead = 4;  // points' records in flight per thread
+        for (int qb = q0 + st0; qb < q1; qb += kAhead * stn) {
+            double4 rec[kAhead];
+            double v[kAhead];
 #pragma unroll
             for (int u = 0; u < kAhead; ++u) {
-                const int q = q0 + u * step + k;
-                const bool in = col && q < np;
-                fa[u] = in ? dyw[q] : 0.0;
-                fb[u] = in ? dy[q] : 0.0;
+                const int q = min(qb + u * stn, q1 - 1);
+                rec[u] = ldg4(&o.pt_rec[q]);
+                v[u] = get(&y[q]);
             }
 #pragma unroll
-            for (int u = 0; u < kAhead; ++u) dmma_8x8x4(c0, c1, fa[u], fb[u]);
+            for (int u = 0; u < kAhead; ++u) {
+                const int q = qb + u * stn;
+                if (q < q1) {
+                    const double ymod = rec[u].w != 0.0 ? __dmul_rn(s.ccoef[(int)rec[u].z], v[u]) : v[u];
+                    const double d = __dsub_rn(rec[u].x, ymod);
+                    dy[q - q0] = d;
+                    dyw[q - q0] = __dmul_rn(d, rec[u].y);
+                }
+            }
         }
-        if (warp == owner) {
-            const double d = (col && k < 3) ? 0.0 - (k == 0 ? ym[0] : k == 1 ? ym[1] : ym[2]) : 0.0;
-            dmma_8x8x4(c0, c1, __dmul_rn(d, __dmul_rn(conw_r, conw_r)), d);
+    };
+    double c0 = 0.0, c1 = 0.0;
+    if (stager) stage(0);
+    __syncthreads();
+    for (int c = 0; c < nchunk; ++c) {
+        if (stager && c + 1 < nchunk) stage(c + 1);
+        if (slice || warp == owner) {
+            const double *dy = buf + (c & 1) * 2 * chunk, *dyw = dy + chunk;
+            const int n = min(chunk, np - c * chunk), step = slice ? 4 * kWarps : 4;
+            constexpr int kAhead = 8;
+            for (int q0 = slice ? 4 * warp : 0; q0 < n; q0 += kAhead * step) {
+                double fa[kAhead], fb[kAhead];
+#pragma unroll
+                for (int u = 0; u < kAhead; ++u) {
+                    const int q = q0 + u * step + k;
+                    const bool in = col && q < n;
+                    fa[u] = in ? dyw[q] : 0.0;
+                    fb[u] = in ? dy[q] : 0.0;
+                }
+#pragma unroll
+                for (int u = 0; u < kAhead; ++u) dmma_8x8x4(c0, c1, fa[u], fb[u]);
+            }
         }
-        if (lane == 4 * m + (m >> 1)) s.red[warp] = (m & 1) ? c1 : c0;
+        __syncthreads();
     }
+    if (warp == owner) {
+        const double d = (col && k < 3) ? 0.0 - (k == 0 ? ym[0] : k == 1 ? ym[1] : ym[2]) : 0.0;
+        dmma_8x8x4(c0, c1, __dmul_rn(d, __dmul_rn(conw_r, conw_r)), d);
+    }
+    if (lane == 4 * m + (m >> 1)) s.red[warp] = (m & 1) ? c1 : c0;
     __syncthreads();
     double chisq = 0.0;
     if (slice)
@@ -1531,30 +1943,37 @@ static __device__ double trial_chisq(const DevObject &o, const DevParams &p, con
 // and point order still stand.
 // Writes alpha (symmetric, stride ld) to dst, beta to dvec; returns chi^2 to
 // every thread.
-template <int NCP, bool MIXED>
+template <int NCP, bool MIXED, bool CL>
 __device__ double evaluate(const DevObject &o, const DevParams &p, const Sh &s, const double *a, bool ready,
                            double *dst, double *dvec, double *rows, double *cstat, int *perm, double conw_r)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const Team<CL> team;
     const int ma = o.ma, mfit = o.mfit, mfp = s.mfp, RS = o.row_stride, CS = ma + 3;
+    double *gpart = rows + scratch_gpart(o.n_points, RS, o.n_curves, ma);
 
-    if (o.cstat_smem) cstat = s.cst;  // stride ma + 3 fits inside rs + 2
+    double *const cstat_slab = cstat;
+    if (o.cstat_smem && !CL) cstat = s.cst;  // stride ma + 3 fits inside rs + 2
     tmark(p, s, T_REST);
-    if (!ready) evaluation_setup<MIXED>(o, p, s, a, perm);
+    if (!ready)
+        evaluation_setup<MIXED, CL>(o, p, s, a, rows, perm);
+    else if (CL)
+        team.sync();  // every CTA has read the trial's brightness, whose place the rows take
     if constexpr (MIXED)
-        brightness_rows_mixed<NCP>(o, s, rows, perm);
+        brightness_rows_mixed<NCP, CL>(o, s, rows, perm);
     else
         if (o.n_coef == NCP - 7)
-            brightness_rows<NCP, true>(o, s, rows, perm);
+            brightness_rows<NCP, true, CL>(o, s, rows, perm);
         else
-            brightness_rows<NCP, false>(o, s, rows, perm);
-    // the tile phase reads the rows back through the bulk-copy (async) proxy
-    asm volatile("fence.proxy.async.global;" ::: "memory");
-    __syncthreads();
+            brightness_rows<NCP, false, CL>(o, s, rows, perm);
+    // the tile phase of one CTA reads the rows back through the bulk-copy
+    // (async) proxy
+    if constexpr (!CL) asm volatile("fence.proxy.async.global;" ::: "memory");
+    team.sync();
     tmark(p, s, T_SWEEP);
 
     // per relative curve: column sums, 1/sum(ymod) and the renormalisation coefficient
-    for (int c = warp; c < o.n_curves; c += kWarps) {
+    for (int c = warp + kWarps * team.rank(); c < o.n_curves; c += kWarps * team.size()) {
         if (!o.curve_rel[c]) continue;
         const int p0 = o.curve_start[c], p1 = o.curve_start[c + 1];
         // columns lane, lane + 32, lane + 64 (ma + 1 <= 90); the rows come from
@@ -1568,7 +1987,7 @@ __device__ double evaluate(const DevObject &o, const DevParams &p, const Sh &s, 
                 const bool ok = q0 + u < p1;
                 const double *r = rows + (size_t)(ok ? q0 + u : p0) * RS;
 #pragma unroll
-                for (int j = 0; j < 3; ++j) v[u][j] = (ok && lane + 32 * j <= ma) ? r[lane + 32 * j] : 0.0;
+                for (int j = 0; j < 3; ++j) v[u][j] = (ok && lane + 32 * j <= ma) ? team.load(&r[lane + 32 * j]) : 0.0;
             }
 #pragma unroll
             for (int u = 0; u < kStep; ++u)
@@ -1579,12 +1998,32 @@ __device__ double evaluate(const DevObject &o, const DevParams &p, const Sh &s, 
         for (int j = 0; j < 3; ++j)
             if (lane + 32 * j <= ma) cstat[(size_t)c * CS + lane + 32 * j] = sum[j];
         __syncwarp();
-        if (lane == 0) {
-            renormalise_curve(o, s, c, cstat[(size_t)c * CS + ma]);
-        }
+        if (!CL && lane == 0) renormalise_curve(s, c, cstat[(size_t)c * CS + ma], o.curve_sig[c], p1 - p0);
     }
-    __syncthreads();
+    team.sync();
+    if constexpr (CL) {
+        // the curves of the other CTAs
+        if (o.cstat_smem) {
+            cstat = s.cst;
+            for (int i = tid; i < o.n_curves * CS; i += kThreads) cstat[i] = team.load(&cstat_slab[i]);
+        }
+        for (int c = tid; c < o.n_curves; c += kThreads)
+            if (o.curve_rel[c])
+                renormalise_curve(s, c, team.load(&cstat_slab[(size_t)c * CS + ma]), o.curve_sig[c],
+                                  o.curve_start[c + 1] - o.curve_start[c]);
+        __syncthreads();
+    }
     tmark(p, s, T_CSTAT);
+    if constexpr (CL) {
+        if (team.size() == 8)
+            normal_matrix_team<8>(o, s, rows, cstat, dst, dvec, gpart, conw_r);
+        else if (team.size() == 4)
+            normal_matrix_team<4>(o, s, rows, cstat, dst, dvec, gpart, conw_r);
+        else
+            normal_matrix_team<2>(o, s, rows, cstat, dst, dvec, gpart, conw_r);
+        tmark(p, s, T_TSYRK);
+        return s.scal[S_TRIAL];
+    }
 
     SyrkAcc acc;
     syrk_init(mfit, s.tr, acc);
@@ -1775,62 +2214,15 @@ __device__ double evaluate(const DevObject &o, const DevParams &p, const Sh &s, 
 
     // convexity regularisation pseudo-points (mrqcof_curve1_last_opt, Start.cu:2539-2612)
     {
-        const int nc = o.n_coef, nf = o.n_fac;
         double ym[3];
         moment_sums(o, s, ym);
-        // raw derivative d ym_i / d a_k for shape coefficient k = tid: groups
-        // of nc threads take consecutive facet ranges, their partial sums
-        // (staged in the idle tile buffer) are added in group order
-        double dk[3] = {0, 0, 0};
-        {
-            const int ngrp = max(1, min(kThreads / nc, (s.tr * mfp) / (3 * nc)));
-            const int per = (nf + ngrp - 1) / ngrp;
-            const int grp = tid / nc, k = tid - grp * nc;
-            if (grp < ngrp) {
-                double pk[3] = {0, 0, 0};
-                const int fe = min(nf, (grp + 1) * per);
-                for (int fi = grp * per; fi < fe; ++fi) {
-                    const double4 fr = s.F[fi];
-                    const double y = __ldg(o.ysh + (size_t)fi * o.ncp + k);
-                    pk[0] += (fr.w * fr.x) * y;
-                    pk[1] += (fr.w * fr.y) * y;
-                    pk[2] += (fr.w * fr.z) * y;
-                }
-#pragma unroll
-                for (int i = 0; i < 3; ++i) s.T[(grp * 3 + i) * nc + k] = pk[i];
-            }
-            __syncthreads();
-            if (tid < nc)
-                for (int g2 = 0; g2 < ngrp; ++g2)
-#pragma unroll
-                    for (int i = 0; i < 3; ++i) dk[i] += s.T[(g2 * 3 + i) * nc + tid];
-            __syncthreads();
-        }
-        const double wps = conw_r * conw_r;
-        for (int idx = tid; idx < kTile * mfp; idx += kThreads) {
-            s.T[idx] = 0.0;
-            s.TW[idx] = 0.0;
-        }
-        __syncthreads();
-        if (tid < nc) {
-            int slot = -1;  // fit slot of parameter tid + 1, if fitted
-            for (int j = 0; j < mfit; ++j)
-                if (s.fidx[j] == tid + 1) slot = j;
-            if (slot >= 0)
-                for (int i = 0; i < 3; ++i) {
-                    s.T[i * mfp + slot] = dk[i];
-                    s.TW[i * mfp + slot] = dk[i] * wps;
-                }
-        }
-        if (tid < 3) {
-            const double dy = 0.0 - ym[tid];
-            s.T[tid * mfp + mfit] = dy;
-            s.TW[tid * mfp + mfit] = dy * wps;
-        }
+        double dk[3];
+        pseudo_derivatives(o, s, dk);
+        stage_pseudo_rows(o, s, ym, dk, conw_r);
         __syncthreads();
         syrk_update(s, 3, acc);
     }
-    syrk_store(s, mfit, acc, dst, dvec, rows + scratch_gpart(o.n_points, RS, o.n_curves, ma));
+    syrk_store(s, mfit, acc, dst, dvec, gpart);
     tmark(p, s, T_PSEUDO);
     if (p.phase_cycles && tid == 0) atomicAdd(&p.phase_cycles[T_NPHASE], 1ull);
     return s.scal[S_TRIAL];
@@ -2120,7 +2512,38 @@ static __device__ int gauss_jordan(const Sh &s, int n)
 
 // One (frequency, pole) fit, the whole LM loop, by the CTA; its result to
 // out[item].  o and p are the fit's object and constants.
+// A team's kernel keeps the object, the constants and the shared-memory layout
+// in shared memory and calls its phases instead of inlining them: inlined, the
+// live state around the team update pushed spills into every phase (brightness
+// sweep +60 %).
+struct TeamShared {
+    DevObject o;
+    DevParams p;
+    Sh s;
+};
+
 template <int NCP, bool MIXED>
+static __device__ __noinline__ double evaluate_call(const DevObject &o, const DevParams &p, const Sh &s, const double *a,
+                                                    bool ready, double *dst, double *dvec, double *rows, double *cstat,
+                                                    int *perm, double conw_r)
+{
+    return evaluate<NCP, MIXED, true>(o, p, s, a, ready, dst, dvec, rows, cstat, perm, conw_r);
+}
+
+template <bool MIXED>
+static __device__ __noinline__ double trial_call(const DevObject &o, const DevParams &p, const Sh &s, double *rows,
+                                                 int *perm, double conw_r)
+{
+    return trial_chisq<MIXED, true>(o, p, s, rows, perm, conw_r);
+}
+
+template <int kMaxN>
+static __device__ __noinline__ int solve_call(const Sh &s, int n)
+{
+    return gauss_jordan<kMaxN>(s, n);
+}
+
+template <int NCP, bool MIXED, bool CL>
 __device__ __forceinline__ void fit_one(const DevObject &o, const DevParams &p, const Sh &s, const FitItem it,
                                         int item, FitOut *out, double *rows, int *status)
 {
@@ -2169,7 +2592,11 @@ __device__ __forceinline__ void fit_one(const DevObject &o, const DevParams &p, 
         // alpha and beta at the current parameters: at the start, and after an
         // accepted step -- only now, so a fit that ends with one does without
         if (first || moved) {
-            const double oc = evaluate<NCP, MIXED>(o, p, s, s.a, moved, s.alpha, s.beta, rows, cstat, perm, p.conw_r);
+            double oc;
+            if constexpr (CL)
+                oc = evaluate_call<NCP, MIXED>(o, p, s, s.a, moved, s.alpha, s.beta, rows, cstat, perm, p.conw_r);
+            else
+                oc = evaluate<NCP, MIXED, CL>(o, p, s, s.a, moved, s.alpha, s.beta, rows, cstat, perm, p.conw_r);
             moved = false;
             if (first) {
                 if (tid == 0) {
@@ -2191,14 +2618,23 @@ __device__ __forceinline__ void fit_one(const DevObject &o, const DevParams &p, 
         __syncthreads();
         tmark(p, s, T_REST);
         // mfit <= ma = n_coef + 8 <= NCP + 8 (and < kMaxFit)
-        const int err = gauss_jordan<(NCP + 8 < kMaxFit ? NCP + 8 : kMaxFit)>(s, mfit);
+        constexpr int kMaxN = NCP + 8 < kMaxFit ? NCP + 8 : kMaxFit;
+        int err;
+        if constexpr (CL)
+            err = solve_call<kMaxN>(s, mfit);
+        else
+            err = gauss_jordan<kMaxN>(s, mfit);
         tmark(p, s, T_SOLVE);
         if (err == 0 || err == 2) {
             if (tid < mfit) s.atry[s.fidx[tid]] = s.a[s.fidx[tid]] + s.da[tid];
             if (err == 2 && tid == 0) s.ctl[C_STATUS] |= kStatusSingular;
         }
         __syncthreads();
-        const double chisq = trial_chisq<MIXED>(o, p, s, rows, perm, p.conw_r);
+        double chisq;
+        if constexpr (CL)
+            chisq = trial_call<MIXED>(o, p, s, rows, perm, p.conw_r);
+        else
+            chisq = trial_chisq<MIXED, CL>(o, p, s, rows, perm, p.conw_r);
         // accept / reject (mrqmin_2_end, Start.cu:300-392)
         const bool accept = chisq < s.scal[S_OCHISQ];
         __syncthreads();
@@ -2249,8 +2685,8 @@ __device__ __forceinline__ void fit_one(const DevObject &o, const DevParams &p, 
         __syncthreads();
     }
 
-    // per-fit result (CudaCalculateFinishPole, Start.cu:5056-5125)
-    if (tid == 0) {
+    // per-fit result (CudaCalculateFinishPole, Start.cu:5056-5125), alike in all CTAs of a team
+    if (tid == 0 && Team<CL>().rank() == 0) {
         double dd = s.scal[S_CHCK] * 100.0 * (1.0 / s.scal[S_AREA]);
         if (isnan(dd)) dd = 1.0;
         const double la = (180 / kPi) * s.a[nc + 2];
@@ -2275,9 +2711,9 @@ __device__ __forceinline__ void fit_one(const DevObject &o, const DevParams &p, 
     }
 }
 
-template <int NCP, bool MIXED, bool BATCH>
+template <int NCP, bool MIXED, bool BATCH, bool CL>
 __global__ void __launch_bounds__(kThreads, 1)
-fit_kernel(DevObject o, DevParams p, const FitItem *items, int n_items, int *queue, FitOut *out,
+fit_kernel(DevObject obj, DevParams prm, const FitItem *items, int n_items, int *queue, FitOut *out,
            double *scratch, size_t scratch_per_cta, int *status, EvalOut ev, int mode, const DevObject *objs,
            const DevParams *prms)
 {
@@ -2287,11 +2723,24 @@ fit_kernel(DevObject o, DevParams p, const FitItem *items, int n_items, int *que
     __shared__ DevObject s_obj;
     __shared__ DevParams s_prm;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Sh s;
-    carve_bytes(o.n_fac, o.mfit, o.ncp, o.n_curves, o.row_stride, o.tile_rows, o.cstat_smem, MIXED ? 1 : 0, &s,
-                smem_raw);
     const int tid = threadIdx.x;
-    double *rows = scratch + (size_t)blockIdx.x * scratch_per_cta;
+    const Team<CL> team;
+    Sh own;
+    carve_bytes(obj.n_fac, obj.mfit, obj.ncp, obj.n_curves, obj.row_stride, obj.tile_rows, obj.cstat_smem, MIXED ? 1 : 0,
+                &own, smem_raw);
+    __shared__ TeamShared s_team;  // used by teams only
+    if constexpr (CL) {
+        if (tid == 0) {
+            s_team.o = obj;
+            s_team.p = prm;
+            s_team.s = own;
+        }
+        __syncthreads();
+    }
+    const DevObject &o = *[&] { if constexpr (CL) return &s_team.o; else return &obj; }();
+    const DevParams &p = *[&] { if constexpr (CL) return &s_team.p; else return &prm; }();
+    const Sh &s = *[&] { if constexpr (CL) return &s_team.s; else return &own; }();
+    double *rows = scratch + (size_t)team.index() * scratch_per_cta;
 
     if constexpr (!BATCH) {
         for (int f = tid; f < o.n_fac; f += kThreads) s.F[f] = ldg4(&o.facet[f]);
@@ -2322,7 +2771,12 @@ fit_kernel(DevObject o, DevParams p, const FitItem *items, int n_items, int *que
             int *perm = reinterpret_cast<int *>(rows + scratch_perm(o.n_points, o.row_stride, o.n_curves, ma));
             for (int q = tid; q <= ma; q += kThreads) s.a[q] = ev.a[q];
             __syncthreads();
-            double chisq = evaluate<NCP, MIXED>(o, p, s, s.a, false, s.alpha, s.beta, rows, cstat, perm, p.conw_r);
+            double chisq;
+            if constexpr (CL)
+                chisq = evaluate_call<NCP, MIXED>(o, p, s, s.a, false, s.alpha, s.beta, rows, cstat, perm, p.conw_r);
+            else
+                chisq = evaluate<NCP, MIXED, CL>(o, p, s, s.a, false, s.alpha, s.beta, rows, cstat, perm, p.conw_r);
+            if (team.rank() != 0) return;
             for (int idx = tid; idx < mfit * mfit; idx += kThreads) {
                 const int j = idx / mfit, k = idx - j * mfit;
                 ev.alpha[idx] = s.alpha[j * ld + k];
@@ -2338,9 +2792,29 @@ fit_kernel(DevObject o, DevParams p, const FitItem *items, int n_items, int *que
 
     int cur = -1;  // batch: the object whose tables are loaded
     for (;;) {
-        if (tid == 0) s.ctl[C_ITEM] = atomicAdd(queue, 1);
-        __syncthreads();
-        const int item = s.ctl[C_ITEM];
+        int item;
+        if constexpr (CL) {
+            // the team's first CTA takes the next item and hands it on through
+            // the slab; all stop once any of them met a timeout
+            int *hand = reinterpret_cast<int *>(rows);
+            team.sync();  // the previous fit's slab is free
+            if (tid == 0 && team.rank() == 0) {
+                hand[0] = atomicAdd(queue, 1);
+                hand[1] = 0;
+            }
+            team.sync();
+            if (tid == 0 && s.ctl[C_TIMEOUT]) {
+                atomicOr(&hand[1], 1);
+                atomicOr(status, kStatusTimeout);
+            }
+            team.sync();
+            item = team.load(&hand[1]) ? n_items : team.load(&hand[0]);
+            team.sync();
+        } else {
+            if (tid == 0) s.ctl[C_ITEM] = atomicAdd(queue, 1);
+            __syncthreads();
+            item = s.ctl[C_ITEM];
+        }
         if (item >= n_items) break;
         const FitItem it = items[item];
         if constexpr (BATCH) {
@@ -2357,12 +2831,12 @@ fit_kernel(DevObject o, DevParams p, const FitItem *items, int n_items, int *que
                 __syncthreads();
                 cur = k;
             }
-            fit_one<NCP, MIXED>(s_obj, s_prm, s, it, item, out, rows, status);
+            fit_one<NCP, MIXED, CL>(s_obj, s_prm, s, it, item, out, rows, status);
         } else {
-            fit_one<NCP, MIXED>(o, p, s, it, item, out, rows, status);
+            fit_one<NCP, MIXED, CL>(o, p, s, it, item, out, rows, status);
         }
         __syncthreads();
-        if (s.ctl[C_TIMEOUT]) break;  // a bulk copy never completed: stop taking items
+        if (!CL && s.ctl[C_TIMEOUT]) break;  // a bulk copy never completed: stop taking items
     }
     // after a timeout, give any copy still in flight a bounded chance to land
     // before the CTA's shared memory is released

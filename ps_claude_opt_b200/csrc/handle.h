@@ -57,6 +57,8 @@ struct ps_gpu {
     int device = 0;
     int n_sm = 0;
     cudaStream_t stream = nullptr;
+    cudaStream_t side = nullptr;   // the teams of a launch that has single CTAs too
+    cudaEvent_t fork = nullptr, join = nullptr;
     int quirks = 0;
     int precision = PS_PRECISION_FP64;  // applies from the next configure
     // prepare-time inputs
@@ -70,7 +72,7 @@ struct ps_gpu {
     psb::DevParams prm{};
     int ctas_per_sm = 0;
     psb::DevBuf<double4> facet, pt_a, pt_b, pt_rec;
-    psb::DevBuf<double> ysh, pt_w, curve_sig, cg_first, scratch, eval_buf;
+    psb::DevBuf<double> ysh, ysh_t, pt_w, curve_sig, cg_first, scratch, eval_buf;
     psb::DevBuf<float> ysh32;
     psb::DevBuf<int> pt_curve, curve_start, curve_rel, fidx, queue, status;
     psb::DevBuf<psb::FitItem> items;

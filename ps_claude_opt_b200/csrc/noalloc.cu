@@ -35,6 +35,8 @@
 //     objects, so slower than ps_gpu_fit_items, never different).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstring>
 
@@ -78,6 +80,13 @@ __global__ void pack_points(int np, const int *curve_start, int n_curves, const 
     pw[q] = w;
     pcur[q] = c;
     prec[q] = make_double4(pt_b[q].w, w, (double)c, (double)curve_rel[c]);
+}
+
+// The basis transposed: yt[k][f] = y[f][k].
+__global__ void transpose_basis(int nf, int nc, int ncp, const double *y, double *yt)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < nf * nc) yt[i] = y[(size_t)(i % nf) * ncp + i / nf];
 }
 
 struct Carver {
@@ -185,7 +194,9 @@ extern "C" ps_status ps_fit_items_noalloc(
     const size_t o_fidx = cv.take<int>(mfit), o_cg = cv.take<double>(nc);
     const size_t o_items = cv.take<psb::FitItem>(n), o_out = cv.take<psb::FitOut>(n);
     const size_t o_ctl = cv.take<int>(2);
-    const size_t o_scratch = cv.off;
+    const size_t o_bare = cv.off;
+    const size_t o_ysht = cv.take<double>((size_t)nfac * nc);
+    size_t o_scratch = cv.off;
 
     psb::DevObject o{};
     o.n_points = ndata;
@@ -199,10 +210,15 @@ extern "C" ps_status ps_fit_items_noalloc(
     o.tile_rows = tile_rows;
     o.cstat_smem = cstat_smem;
     const size_t per_cta = psb::fit_scratch_doubles(o) * sizeof(double);
+    // the transposed basis is left out where it would cost a scratch slab
+    const bool with_t = o_scratch <= kNoAllocArenaBytes &&
+                        (kNoAllocArenaBytes - o_scratch) / per_cta == (kNoAllocArenaBytes - o_bare) / per_cta;
+    if (!with_t) o_scratch = o_bare;
     if (o_scratch + per_cta > kNoAllocArenaBytes)
         return psb_fail(PS_ERR_ARG, "ps_fit_items_noalloc: object and items exceed the 64 MiB arena");
     o.facet = reinterpret_cast<const double4 *>(arena + o_facet);
     o.ysh = reinterpret_cast<const double *>(arena + o_ysh);
+    o.ysh_t = with_t ? reinterpret_cast<const double *>(arena + o_ysht) : nullptr;
     o.pt_a = reinterpret_cast<const double4 *>(arena + o_pa);
     o.pt_b = reinterpret_cast<const double4 *>(arena + o_pb);
     o.pt_w = reinterpret_cast<const double *>(arena + o_pw);
@@ -224,6 +240,11 @@ extern "C" ps_status ps_fit_items_noalloc(
     NA_CUDA(cudaMemsetAsync(arena + o_ysh, 0, (size_t)nfac * ncp * sizeof(double), s));
     NA_CUDA(cudaMemcpy2DAsync(arena + o_ysh, ncp * sizeof(double), shape->d_sphere, nc * sizeof(double),
                               nc * sizeof(double), nfac, h2d, s));
+    if (with_t) {
+        transpose_basis<<<(nfac * nc + 255) / 256, 256, 0, s>>>(nfac, nc, ncp, o.ysh,
+                                                                reinterpret_cast<double *>(arena + o_ysht));
+        NA_CUDA(cudaGetLastError());
+    }
     // point records {t, ee} and {ee0, brightness}
     NA_CUDA(cudaMemcpy2DAsync(arena + o_pa, sizeof(double4), tim, sizeof(double), sizeof(double), ndata, h2d, s));
     NA_CUDA(cudaMemcpy2DAsync(arena + o_pa + sizeof(double), sizeof(double4), ee, 3 * sizeof(double),
@@ -286,14 +307,17 @@ extern "C" ps_status ps_fit_items_noalloc(
     const int per_sm = psb::fit_ctas_per_sm(o);
     if (per_sm < 1) return psb_fail(PS_ERR_CUDA, "ps_fit_items_noalloc: fit kernel cannot be resident");
     const size_t fit_scratch = (kNoAllocArenaBytes - o_scratch) / per_cta;
-    int n_ctas = per_sm * n_sm;
-    if ((size_t)n_ctas > fit_scratch) n_ctas = (int)fit_scratch;
-    if (n_ctas > n) n_ctas = n;
+    const psb::FitPlan pl = psb::plan_fits(o, n, per_sm * n_sm, (int)std::min<size_t>(fit_scratch, INT_MAX), false);
     int *ctl = reinterpret_cast<int *>(arena + o_ctl);
-    int e = psb::launch_fits(o, p, reinterpret_cast<const psb::FitItem *>(arena + o_items), n, ctl,
-                             reinterpret_cast<psb::FitOut *>(arena + o_out),
-                             reinterpret_cast<double *>(arena + o_scratch), per_cta / sizeof(double), n_ctas,
-                             ctl + 1, s);
+    const auto *d_items = reinterpret_cast<const psb::FitItem *>(arena + o_items);
+    auto *d_out = reinterpret_cast<psb::FitOut *>(arena + o_out);
+    auto *scratch = reinterpret_cast<double *>(arena + o_scratch);
+    const size_t per_slab = per_cta / sizeof(double);
+    int e;
+    if (pl.team_items > 0)
+        e = psb::launch_fit_teams(o, p, d_items, n, ctl, d_out, scratch, per_slab, pl.teams, pl.team_size, ctl + 1, s);
+    else
+        e = psb::launch_fits(o, p, d_items, n, ctl, d_out, scratch, per_slab, pl.main_ctas, ctl + 1, s);
     if (e) return psb_fail_cuda(e, "ps_fit_items_noalloc: fit kernel launch");
     NA_CUDA(cudaMemcpyAsync(out, arena + o_out, (size_t)n * sizeof(ps_fit_result), cudaMemcpyDeviceToHost, s));
     NA_CUDA(cudaStreamSynchronize(s));
