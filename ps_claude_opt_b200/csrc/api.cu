@@ -51,11 +51,13 @@ extern "C" ps_status ps_gpu_prepare(int32_t device, const double *beta_pole, con
     PSB_CUDA(cudaGetDeviceCount(&ndev));
     if (device < 0 || device >= ndev) return psb_fail(PS_ERR_ARG, "ps_gpu_prepare: no such CUDA device");
     PSB_CUDA(cudaSetDevice(device));
-    cudaDeviceProp prop;
-    PSB_CUDA(cudaGetDeviceProperties(&prop, device));
+    int n_sm = 0, smem_optin = 0;
+    PSB_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, device));
+    PSB_CUDA(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
     ps_gpu *h = new ps_gpu();
     h->device = device;
-    h->n_sm = prop.multiProcessorCount;
+    h->n_sm = n_sm;
+    h->smem_limit = (size_t)smem_optin;
     cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
         delete h;
@@ -165,8 +167,6 @@ extern "C" ps_status ps_gpu_configure(ps_gpu *h, double freq_start, double freq_
     if (mfit < 1) return psb_fail(PS_ERR_ARG, "ps_gpu_configure: no fitted parameters");
     const int ncp = psb::padded_ncoef(nc);
 
-    cudaDeviceProp prop;
-    PSB_CUDA(cudaGetDeviceProperties(&prop, h->device));
     const int mixed = h->precision == PS_PRECISION_MIXED ? 1 : 0;
     if (mixed && ncp > psb::kMaxMixedNcp)
         return psb_fail(PS_ERR_ARG, "ps_gpu_configure: mixed precision is built for n_coef <= 64 (lmax <= 7)");
@@ -175,15 +175,15 @@ extern "C" ps_status ps_gpu_configure(ps_gpu *h, double freq_start, double freq_
     int tile_rows = 32, cstat_smem = 1;
     const int rs = (ma + 2) & ~1;
     size_t smem = psb::fit_smem_bytes(numfac, mfit, ncp, curves->n_curves, rs, tile_rows, cstat_smem, mixed);
-    if (smem > prop.sharedMemPerBlockOptin) {
+    if (smem > h->smem_limit) {
         cstat_smem = 0;
         smem = psb::fit_smem_bytes(numfac, mfit, ncp, curves->n_curves, rs, tile_rows, cstat_smem, mixed);
     }
-    if (smem > prop.sharedMemPerBlockOptin) {
+    if (smem > h->smem_limit) {
         tile_rows = 16;
         smem = psb::fit_smem_bytes(numfac, mfit, ncp, curves->n_curves, rs, tile_rows, cstat_smem, mixed);
     }
-    if (smem > prop.sharedMemPerBlockOptin)
+    if (smem > h->smem_limit)
         return psb_fail(PS_ERR_ARG, "ps_gpu_configure: object too large for shared memory");
 
     std::vector<double4> facet(numfac);

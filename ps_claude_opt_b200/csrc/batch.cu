@@ -412,8 +412,6 @@ extern "C" ps_status ps_gpu_scan_batch(int32_t device, int32_t n_obj, const ps_o
         if (st != PS_OK) return st;
     }
     PSB_CUDA(cudaSetDevice(device));
-    cudaDeviceProp prop;
-    PSB_CUDA(cudaGetDeviceProperties(&prop, device));
     PSB_CUDA(cudaStreamCreateWithFlags(&b.origin, cudaStreamNonBlocking));
     PSB_CUDA(cudaEventCreateWithFlags(&b.fork, cudaEventDisableTiming));
     std::map<int, int> by_ncp;
@@ -430,7 +428,7 @@ extern "C" ps_status ps_gpu_scan_batch(int32_t device, int32_t n_obj, const ps_o
     for (Group &g : b.groups) {
         PSB_CUDA(cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking));
         PSB_CUDA(cudaEventCreateWithFlags(&g.join, cudaEventDisableTiming));
-        ps_status st = plan_group(b, g, prop.sharedMemPerBlockOptin, report);
+        ps_status st = plan_group(b, g, b.h[0]->smem_limit, report);
         if (st != PS_OK) return st;
     }
     report += "]";

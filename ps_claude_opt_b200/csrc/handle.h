@@ -56,6 +56,7 @@ cudaError_t upload(DevBuf<T> &b, const std::vector<T> &v, cudaStream_t s)
 struct ps_gpu {
     int device = 0;
     int n_sm = 0;
+    size_t smem_limit = 0;  // shared memory one block may have
     cudaStream_t stream = nullptr;
     cudaStream_t side = nullptr;   // the teams of a launch that has single CTAs too
     cudaEvent_t fork = nullptr, join = nullptr;

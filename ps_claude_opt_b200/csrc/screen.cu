@@ -524,7 +524,7 @@ extern "C" ps_status ps_screen_features(int32_t device, int32_t n_points, const 
                                                          : std::cos(2.0 * 3.14159265358979323846 * j / 32.0);
     SC_CUDA(cudaSetDevice(device));
     unsigned char *d = nullptr;
-    cudaError_t e = cudaMalloc(&d, off);
+    cudaError_t e = (cudaError_t)psb_pool_alloc(device, (void **)&d, off, nullptr);
     if (e == cudaSuccess) e = cudaMemcpy(d, host.data(), in_bytes, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) {
         auto *k = narrow ? features_kernel<true> : features_kernel<false>;
@@ -535,7 +535,7 @@ extern "C" ps_status ps_screen_features(int32_t device, int32_t n_points, const 
     }
     if (e == cudaSuccess)
         e = cudaMemcpy(features, d + o_out, sizeof(float) * (size_t)n_freq * kFeatures, cudaMemcpyDeviceToHost);
-    cudaFree(d);
+    psb_pool_free(d, nullptr);
     if (e != cudaSuccess) return psb_fail_cuda(e, "ps_screen_features");
     return PS_OK;
 }
