@@ -312,7 +312,23 @@ ps_status ps_column_sum(int32_t rows, int32_t cols, const float *x, float *out, 
    not null, receives the BF16 copy. */
 ps_status ps_adam_step(int64_t n, float *w, const float *grad, float *m, float *v, float lr,
                        float beta1, float beta2, float eps, int32_t step, void *wb, void *stream);
+/* The same step on up to 32 tensors (n[i] values each) in one launch. */
+ps_status ps_adam_steps(int32_t count, const int64_t *n, float *const *w, const float *const *grad,
+                        float *const *m, float *const *v, void *const *wb, float lr, float beta1,
+                        float beta2, float eps, int32_t step, void *stream);
 ps_status ps_to_bf16(int64_t n, const float *x, void *y, void *stream);
+/* The whole network (layers of widths sizes[0..n_layers], weights w[l]
+   BF16 [sizes[l+1]][sizes[l]], ReLU between layers).  Forward: h[0] holds the
+   BF16 input [rows][sizes[0]]; h[1..n_layers-1] receive the BF16 activations,
+   hf[l] the FP32 output of layer l (hf of a hidden layer may be null).
+   Backward: dz[n_layers-1] holds the FP32 gradient of the outputs; dz[l], dzb[l]
+   receive each layer's output gradient (FP32, BF16), gw[l], gb[l] the weight
+   and bias gradients; h and hf are the forward pass's. */
+ps_status ps_mlp_forward(int32_t n_layers, const int32_t *sizes, int32_t rows, const void *const *w,
+                         const float *const *bias, void *const *h, float *const *hf, void *stream);
+ps_status ps_mlp_backward(int32_t n_layers, const int32_t *sizes, int32_t rows, const void *const *w,
+                          const void *const *h, const float *const *hf, float *const *dz,
+                          void *const *dzb, float *const *gw, float *const *gb, void *stream);
 
 /* Host shape setup (trifac.c, areanorm.c, sphfunc.c, ellfit.c of the
    reference): facet normals, areas, Laplace basis and the ellipsoid fit. */

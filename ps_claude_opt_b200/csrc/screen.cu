@@ -334,56 +334,269 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// C[m][n] (+)= sum_k A(m, k) B(k, n) (+ bias[n]) (ReLU), A(m, k) = A[m sam + k sak],
-// B(k, n) = B[k sbk + n sbn], BF16 operands on the tensor cores, FP32
-// accumulation.  A block of 4 warps computes a 64 x 32 tile; operands are
-// read element by element with bounds checks, so any strides (transposes)
-// and any sizes work.
-constexpr int kGemmTM = 64, kGemmTN = 32;
+// One product C[m][n] (+)= sum_k A(m, k) B(k, n) (+ bias[n]) (ReLU) (gated),
+// A(m, k) = A[m sam + k sak], B(k, n) = B[k sbk + n sbn], BF16 operands on the
+// tensor cores, FP32 accumulation.  gate: results where gate[m][n] <= 0 become
+// zero (a ReLU's backward pass).
+struct Gemm {
+    int M, N, K;
+    const __nv_bfloat16 *A, *B;
+    long sam, sak, sbk, sbn;
+    float *C;
+    int ldc, accumulate;
+    const float *bias;
+    int relu;
+    const float *gate;
+    int ldg;
+    __nv_bfloat16 *Cb;
+    int ldcb;
+    int a_vec, b_vec;    // 16-byte loads along the contiguous direction are aligned
+    int form, tiles_n, tiles;  // filled by the launch
+};
 
-__global__ void __launch_bounds__(128) gemm_bf16_kernel(int M, int N, int K, const __nv_bfloat16 *A, long sam,
-                                                        long sak, const __nv_bfloat16 *B, long sbk, long sbn,
-                                                        float *C, int ldc, int accumulate, const float *bias,
-                                                        int relu, __nv_bfloat16 *Cb, int ldcb)
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const __nv_bfloat16 *p, bool trans)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    const int m0 = blockIdx.y * kGemmTM + warp * 16;
-    const int n0 = blockIdx.x * kGemmTN;
-    const __nv_bfloat16 zero = __float2bfloat16(0.0f);
-    auto ld_a = [&](int m, int k) { return (m < M && k < K) ? A[(long)m * sam + (long)k * sak] : zero; };
-    auto ld_b = [&](int k, int n) { return (k < K && n < N) ? B[(long)k * sbk + (long)n * sbn] : zero; };
-    float acc[4][4];
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    if (trans)
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(a));
+    else
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(a));
+}
+
+// Eight operand elements along `in` (stride s_in) at outer index `out` (stride
+// s_out), zeros outside n_in x n_out.
+__device__ __forceinline__ uint4 load8(const __nv_bfloat16 *base, long s_in, long s_out, int in, int out, int n_in,
+                                       int n_out, bool vec)
+{
+    if (out < n_out && vec && in + 8 <= n_in)
+        return *reinterpret_cast<const uint4 *>(base + (long)out * s_out + in);
+    __nv_bfloat16 v[8];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
-    for (int k0 = 0; k0 < K; k0 += 16) {
-        uint32_t a[4];
-        a[0] = pack_bf16(ld_a(m0 + g, k0 + 2 * t), ld_a(m0 + g, k0 + 2 * t + 1));
-        a[1] = pack_bf16(ld_a(m0 + g + 8, k0 + 2 * t), ld_a(m0 + g + 8, k0 + 2 * t + 1));
-        a[2] = pack_bf16(ld_a(m0 + g, k0 + 2 * t + 8), ld_a(m0 + g, k0 + 2 * t + 9));
-        a[3] = pack_bf16(ld_a(m0 + g + 8, k0 + 2 * t + 8), ld_a(m0 + g + 8, k0 + 2 * t + 9));
+    for (int e = 0; e < 8; ++e)
+        v[e] = (out < n_out && in + e < n_in) ? base[(long)out * s_out + (long)(in + e) * s_in] : __float2bfloat16(0.0f);
+    uint4 r;
+    r.x = pack_bf16(v[0], v[1]);
+    r.y = pack_bf16(v[2], v[3]);
+    r.z = pack_bf16(v[4], v[5]);
+    r.w = pack_bf16(v[6], v[7]);
+    return r;
+}
+
+constexpr int kGemmThreads = 256;
+constexpr int kGemmSmem = 32768;  // partial sums; the operand stages take less
+
+// One BM x BN tile by 8 warps: a warp computes a WM x WN block over every KS-th
+// k-step of 16; with KS > 1 the partial sums meet in shared memory.  Stages of
+// BK along k: global loads of the next stage are in flight under this one's
+// MMAs.  An operand lies in shared memory as it does in global memory
+// (contiguous along k, or transposed: AT, BT) and ldmatrix turns it.
+//
+// The network's products are small (256 x 256 x a few thousand): what bounds
+// them is latency, not the tensor cores, so tiles are small enough to give the
+// SMs one each, and where k is long and the tiles few it is split over the
+// warps (tcgen05 tiles of 128 rows would leave most SMs idle).  Elsewhere each
+// result is one chain of k-steps: a split would round hidden activations to
+// other BF16 values.
+// Measured cold, 256-wide layers: 5000 rows forward 42 -> 18 us; batch 1024, a
+// weight gradient and the gradient below it 55 + 15 -> 15 us.
+template <int BM, int BN, int BK, int WM, int WN, int KS, bool AT, bool BT>
+__device__ __forceinline__ void gemm_tile(const Gemm &g, int m0, int n0, unsigned char *smem)
+{
+    static_assert((BM / WM) * (BN / WN) * KS * 32 == kGemmThreads, "8 warps");
+    constexpr int SA = AT ? BM + 8 : BK + 8, SB = BT ? BN + 8 : BK + 8;  // padded rows: no ldmatrix conflicts
+    constexpr int VA = BM * BK / 8 / kGemmThreads, VB = BN * BK / 8 / kGemmThreads;
+    static_assert(((AT ? BK * SA : BM * SA) + (BT ? BK * SB : BN * SB)) * 2 <= kGemmSmem, "stage");
+    static_assert(KS * BM * BN * 4 <= kGemmSmem, "partial sums");
+    __nv_bfloat16 *As = reinterpret_cast<__nv_bfloat16 *>(smem), *Bs = As + (AT ? BK * SA : BM * SA);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int ks = warp % KS, block = warp / KS;
+    const int wm = WM * (block / (BN / WN)), wn = WN * (block % (BN / WN));
+    uint4 ra[VA], rb[VB];
+    auto fetch = [&](int k0) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + 8 * j + g;
-            const uint32_t b0 = pack_bf16(ld_b(k0 + 2 * t, n), ld_b(k0 + 2 * t + 1, n));
-            const uint32_t b1 = pack_bf16(ld_b(k0 + 2 * t + 8, n), ld_b(k0 + 2 * t + 9, n));
-            mma_bf16(acc[j], a, b0, b1);
+        for (int v = 0; v < VA; ++v) {
+            const int i = tid + v * kGemmThreads;
+            if constexpr (AT)
+                ra[v] = load8(g.A, 1, g.sak, m0 + i % (BM / 8) * 8, k0 + i / (BM / 8), g.M, g.K, g.a_vec);
+            else
+                ra[v] = load8(g.A, g.sak, g.sam, k0 + i % (BK / 8) * 8, m0 + i / (BK / 8), g.K, g.M, g.a_vec);
+        }
+#pragma unroll
+        for (int v = 0; v < VB; ++v) {
+            const int i = tid + v * kGemmThreads;
+            if constexpr (BT)
+                rb[v] = load8(g.B, 1, g.sbk, n0 + i % (BN / 8) * 8, k0 + i / (BN / 8), g.N, g.K, g.b_vec);
+            else
+                rb[v] = load8(g.B, g.sbk, g.sbn, k0 + i % (BK / 8) * 8, n0 + i / (BK / 8), g.K, g.N, g.b_vec);
+        }
+    };
+    float acc[WM / 16][WN / 8][4];
+#pragma unroll
+    for (int i = 0; i < WM / 16; ++i)
+#pragma unroll
+        for (int j = 0; j < WN / 8; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.0f;
+    fetch(0);
+    for (int k0 = 0; k0 < g.K; k0 += BK) {
+        __syncthreads();  // the previous stage has been read
+#pragma unroll
+        for (int v = 0; v < VA; ++v) {
+            const int i = tid + v * kGemmThreads;
+            constexpr int W = AT ? BM / 8 : BK / 8;
+            *reinterpret_cast<uint4 *>(As + i / W * SA + i % W * 8) = ra[v];
+        }
+#pragma unroll
+        for (int v = 0; v < VB; ++v) {
+            const int i = tid + v * kGemmThreads;
+            constexpr int W = BT ? BN / 8 : BK / 8;
+            *reinterpret_cast<uint4 *>(Bs + i / W * SB + i % W * 8) = rb[v];
+        }
+        __syncthreads();
+        if (k0 + BK < g.K) fetch(k0 + BK);
+        const int j = lane >> 3, r = lane & 7;
+#pragma unroll
+        for (int kk = 0; kk < BK / 16 / KS; ++kk) {
+            const int k = 16 * (kk * KS + ks);
+            if (k0 + k >= g.K) break;  // zeros from here on
+            uint32_t a[WM / 16][4], b[WN / 16][4];
+#pragma unroll
+            for (int i = 0; i < WM / 16; ++i) {
+                const int m = wm + 16 * i;
+                ldmatrix4(a[i], AT ? As + (k + (j >> 1) * 8 + r) * SA + m + (j & 1) * 8
+                                   : As + (m + (j & 1) * 8 + r) * SA + k + (j >> 1) * 8, AT);
+            }
+#pragma unroll
+            for (int i = 0; i < WN / 16; ++i) {
+                const int n = wn + 16 * i;
+                ldmatrix4(b[i], BT ? Bs + (k + (j & 1) * 8 + r) * SB + n + (j >> 1) * 8
+                                   : Bs + (n + (j >> 1) * 8 + r) * SB + k + (j & 1) * 8, BT);
+            }
+#pragma unroll
+            for (int i = 0; i < WM / 16; ++i)
+#pragma unroll
+                for (int jn = 0; jn < WN / 8; ++jn)
+                    mma_bf16(acc[i][jn], a[i], b[jn >> 1][2 * (jn & 1)], b[jn >> 1][2 * (jn & 1) + 1]);
         }
     }
+    __syncthreads();
+    float *red = reinterpret_cast<float *>(smem) + ks * BM * BN;
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int i = 0; i < WM / 16; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int m = m0 + g + (e >= 2 ? 8 : 0);
-            const int n = n0 + 8 * j + 2 * t + (e & 1);
-            if (m >= M || n >= N) continue;
-            float v = acc[j][e];
-            if (accumulate) v += C[(long)m * ldc + n];
-            if (bias) v += bias[n];
-            if (relu) v = fmaxf(v, 0.0f);
-            if (C) C[(long)m * ldc + n] = v;
-            if (Cb) Cb[(long)m * ldcb + n] = __float2bfloat16(v);
-        }
+        for (int jn = 0; jn < WN / 8; ++jn)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                *reinterpret_cast<float2 *>(red + (wm + 16 * i + 8 * h + (lane >> 2)) * BN + wn + 8 * jn + 2 * (lane & 3)) =
+                    make_float2(acc[i][jn][2 * h], acc[i][jn][2 * h + 1]);
+    __syncthreads();
+    const float *sum = reinterpret_cast<const float *>(smem);
+#pragma unroll
+    for (int e = 0; e < BM * BN / kGemmThreads; ++e) {
+        const int i = tid + e * kGemmThreads, m = m0 + i / BN, n = n0 + i % BN;
+        if (m >= g.M || n >= g.N) continue;
+        float v = 0.0f;
+#pragma unroll
+        for (int w = 0; w < KS; ++w) v += sum[w * BM * BN + i];
+        if (g.accumulate) v += g.C[(long)m * g.ldc + n];
+        if (g.bias) v += g.bias[n];
+        if (g.relu) v = fmaxf(v, 0.0f);
+        if (g.gate && !(g.gate[(long)m * g.ldg + n] > 0.0f)) v = 0.0f;
+        if (g.C) g.C[(long)m * g.ldc + n] = v;
+        if (g.Cb) g.Cb[(long)m * g.ldcb + n] = __float2bfloat16(v);
+    }
+    __syncthreads();
+}
+
+// Up to two independent products in one launch.
+struct GemmPair {
+    Gemm g[2];
+};
+
+// The forms of a product's tiles.
+enum { kForm64, kForm32, kFormSplit };
+constexpr int kFormBM[3] = {64, 32, 32}, kFormBN[3] = {64, 64, 32};
+
+template <bool AT, bool BT>
+__device__ __forceinline__ void gemm_form(const Gemm &g, int t, unsigned char *smem)
+{
+    if (g.form == kForm64)
+        gemm_tile<64, 64, 64, 16, 32, 1, AT, BT>(g, t / g.tiles_n * 64, t % g.tiles_n * 64, smem);
+    else if (g.form == kForm32)
+        gemm_tile<32, 64, 64, 16, 16, 1, AT, BT>(g, t / g.tiles_n * 32, t % g.tiles_n * 64, smem);
+    else
+        gemm_tile<32, 32, 128, 32, 32, 8, AT, BT>(g, t / g.tiles_n * 32, t % g.tiles_n * 32, smem);
+}
+
+__global__ void __launch_bounds__(kGemmThreads) gemm_bf16_kernel(const GemmPair pair)
+{
+    __shared__ __align__(16) unsigned char smem[kGemmSmem];
+    const int second = (int)blockIdx.x >= pair.g[0].tiles;
+    const Gemm &g = pair.g[second];
+    const int t = blockIdx.x - (second ? pair.g[0].tiles : 0);
+    const bool at = g.sak != 1 && g.sam == 1, bt = g.sbk != 1 && g.sbn == 1;
+    if (at && bt)
+        gemm_form<true, true>(g, t, smem);
+    else if (at)
+        gemm_form<true, false>(g, t, smem);
+    else if (bt)
+        gemm_form<false, true>(g, t, smem);
+    else
+        gemm_form<false, false>(g, t, smem);
+}
+
+// Launches one product, or two independent ones (b).  A product takes 64 x 64
+// tiles where they give every SM one (they read half as much per result), else
+// 32 x 64 -- and 32 x 32 with k split over the warps where k is 512 or more:
+// below that the chain of k-steps is as short as the split's own reduction.
+cudaError_t launch_gemm(Gemm a, const Gemm *b, cudaStream_t s)
+{
+    GemmPair p{};
+    p.g[0] = a;
+    if (b) p.g[1] = *b;
+    long tiles = 0;
+    for (int i = 0; i < (b ? 2 : 1); ++i) {
+        Gemm &g = p.g[i];
+        auto count = [&](int f) {
+            return (long)((g.M + kFormBM[f] - 1) / kFormBM[f]) * ((g.N + kFormBN[f] - 1) / kFormBN[f]);
+        };
+        g.form = count(kForm64) >= 148 ? kForm64 : g.K >= 512 ? kFormSplit : kForm32;
+        g.tiles_n = (g.N + kFormBN[g.form] - 1) / kFormBN[g.form];
+        g.tiles = (int)count(g.form);
+        tiles += g.tiles;
+        // the contiguous direction's 16-byte loads: base and outer stride
+        const bool at = g.sak != 1 && g.sam == 1, bt = g.sbk != 1 && g.sbn == 1;
+        const long ao = at ? g.sak : g.sam, bo = bt ? g.sbk : g.sbn;
+        g.a_vec = (at || g.sak == 1) && (uintptr_t)g.A % 16 == 0 && ao % 8 == 0;
+        g.b_vec = (bt || g.sbk == 1) && (uintptr_t)g.B % 16 == 0 && bo % 8 == 0;
+    }
+    if (tiles == 0) return cudaSuccess;
+    gemm_bf16_kernel<<<(unsigned)tiles, kGemmThreads, 0, s>>>(p);
+    return cudaGetLastError();
+}
+
+Gemm make_gemm(int M, int N, int K, const void *A, long sam, long sak, const void *B, long sbk, long sbn, float *C,
+               int ldc, const float *bias, int relu, void *Cb, int ldcb)
+{
+    Gemm g{};
+    g.M = M;
+    g.N = N;
+    g.K = K;
+    g.A = (const __nv_bfloat16 *)A;
+    g.B = (const __nv_bfloat16 *)B;
+    g.sam = sam;
+    g.sak = sak;
+    g.sbk = sbk;
+    g.sbn = sbn;
+    g.C = C;
+    g.ldc = ldc;
+    g.bias = bias;
+    g.relu = relu;
+    g.Cb = (__nv_bfloat16 *)Cb;
+    g.ldcb = ldcb;
+    return g;
 }
 
 // dZ = dH * (Z > 0), as BF16 (the next backward GEMM's operand) and FP32.
@@ -396,30 +609,68 @@ __global__ void relu_backward_kernel(long n, const float *dh, const float *z, fl
     if (dzb) dzb[i] = __float2bfloat16(v);
 }
 
-// db[n] = sum over rows of dZ[r][n] (one thread per column, rows in order).
-__global__ void column_sum_kernel(int rows, int cols, const float *dz, float *db)
+// db[n] = sum over rows of dZ[r][n] for several matrices: blocks of 32 columns,
+// 32 threads a column taking every 32nd row, their sums added in order.  (One
+// thread a column was 60 us for 1024 x 256: a serial chain of loads.)
+struct ColumnSums {
+    struct {
+        int rows, cols, first;  // first: block where the matrix starts
+        const float *x;
+        float *out;
+    } m[16];
+    int n;
+};
+
+__global__ void __launch_bounds__(1024) column_sum_kernel(const ColumnSums a)
 {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= cols) return;
+    __shared__ float part[32][33];
+    int i = 0;
+    while (i + 1 < a.n && (int)blockIdx.x >= a.m[i + 1].first) ++i;
+    const auto &m = a.m[i];
+    const int c = threadIdx.x & 31, r0 = threadIdx.x >> 5;
+    const int n = (blockIdx.x - m.first) * 32 + c;
     float s = 0.0f;
-    for (int r = 0; r < rows; ++r) s += dz[(long)r * cols + n];
-    db[n] = s;
+    if (n < m.cols)
+#pragma unroll 8
+        for (int r = r0; r < m.rows; r += 32) s += m.x[(long)r * m.cols + n];
+    part[r0][c] = s;
+    __syncthreads();
+    if (r0 == 0 && n < m.cols) {
+        float t = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 32; ++k) t += part[k][c];
+        m.out[n] = t;
+    }
 }
 
 // Adam on FP32 master weights, then the BF16 working copy.
-__global__ void adam_kernel(long n, float *w, const float *grad, float *m, float *v, float lr, float b1, float b2,
-                            float eps, float c1, float c2, __nv_bfloat16 *wb)
+struct AdamTensors {
+    struct {
+        long n;
+        int first;  // block where the tensor starts
+        float *w, *m, *v;
+        const float *grad;
+        __nv_bfloat16 *wb;
+    } t[32];
+    int count;
+};
+
+__global__ void __launch_bounds__(256) adam_kernel(const AdamTensors a, float lr, float b1, float b2, float eps, float c1,
+                                                   float c2)
 {
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gr = grad[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * gr;
-    const float vi = b2 * v[i] + (1.0f - b2) * gr * gr;
-    m[i] = mi;
-    v[i] = vi;
-    const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    w[i] = wi;
-    if (wb) wb[i] = __float2bfloat16(wi);
+    int k = 0;
+    while (k + 1 < a.count && (int)blockIdx.x >= a.t[k + 1].first) ++k;
+    const auto &t = a.t[k];
+    const long i = (long)(blockIdx.x - t.first) * 256 + threadIdx.x;
+    if (i >= t.n) return;
+    const float gr = t.grad[i];
+    const float mi = b1 * t.m[i] + (1.0f - b1) * gr;
+    const float vi = b2 * t.v[i] + (1.0f - b2) * gr * gr;
+    t.m[i] = mi;
+    t.v[i] = vi;
+    const float wi = t.w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    t.w[i] = wi;
+    if (t.wb) t.wb[i] = __float2bfloat16(wi);
 }
 
 __global__ void to_bf16_kernel(long n, const float *x, __nv_bfloat16 *y)
@@ -547,11 +798,9 @@ extern "C" ps_status ps_gemm_bf16(int32_t M, int32_t N, int32_t K, const void *A
     if (M < 0 || N < 0 || K < 0 || !A || !B || (!C && !Cb) || (accumulate && !C))
         return psb_fail(PS_ERR_ARG, "ps_gemm_bf16: bad arguments");
     if (M == 0 || N == 0) return PS_OK;
-    dim3 grid((N + kGemmTN - 1) / kGemmTN, (M + kGemmTM - 1) / kGemmTM);
-    gemm_bf16_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(
-        M, N, K, (const __nv_bfloat16 *)A, sam, sak, (const __nv_bfloat16 *)B, sbk, sbn, C, ldc, accumulate, bias,
-        relu, (__nv_bfloat16 *)Cb, ldcb);
-    SC_CUDA(cudaGetLastError());
+    Gemm g = make_gemm(M, N, K, A, sam, sak, B, sbk, sbn, C, ldc, bias, relu, Cb, ldcb);
+    g.accumulate = accumulate;
+    SC_CUDA(launch_gemm(g, nullptr, (cudaStream_t)stream));
     return PS_OK;
 }
 
@@ -568,7 +817,10 @@ extern "C" ps_status ps_column_sum(int32_t rows, int32_t cols, const float *x, f
 {
     if (rows < 0 || cols < 0 || !x || !out) return psb_fail(PS_ERR_ARG, "ps_column_sum: bad arguments");
     if (cols == 0) return PS_OK;
-    column_sum_kernel<<<blocks_for(cols, 128), 128, 0, (cudaStream_t)stream>>>(rows, cols, x, out);
+    ColumnSums a{};
+    a.n = 1;
+    a.m[0] = {rows, cols, 0, x, out};
+    column_sum_kernel<<<blocks_for(cols, 32), 1024, 0, (cudaStream_t)stream>>>(a);
     SC_CUDA(cudaGetLastError());
     return PS_OK;
 }
@@ -578,11 +830,105 @@ extern "C" ps_status ps_adam_step(int64_t n, float *w, const float *grad, float 
 {
     if (n < 0 || !w || !grad || !m || !v || step < 1) return psb_fail(PS_ERR_ARG, "ps_adam_step: bad arguments");
     if (n == 0) return PS_OK;
+    const int64_t sizes[1] = {n};
+    float *ws[1] = {w}, *ms[1] = {m}, *vs[1] = {v};
+    const float *gs[1] = {grad};
+    void *wbs[1] = {wb};
+    return ps_adam_steps(1, sizes, ws, gs, ms, vs, wbs, lr, beta1, beta2, eps, step, stream);
+}
+
+extern "C" ps_status ps_adam_steps(int32_t count, const int64_t *n, float *const *w, const float *const *grad,
+                                   float *const *m, float *const *v, void *const *wb, float lr, float beta1,
+                                   float beta2, float eps, int32_t step, void *stream)
+{
+    if (count < 0 || count > 32 || (count > 0 && (!n || !w || !grad || !m || !v || !wb)) || step < 1)
+        return psb_fail(PS_ERR_ARG, "ps_adam_steps: bad arguments (at most 32 tensors)");
+    AdamTensors a{};
+    long blocks = 0;
+    for (int i = 0; i < count; ++i) {
+        if (n[i] < 0 || (n[i] > 0 && (!w[i] || !grad[i] || !m[i] || !v[i])))
+            return psb_fail(PS_ERR_ARG, "ps_adam_steps: bad arguments (null tensor)");
+        if (n[i] == 0) continue;
+        auto &t = a.t[a.count++];
+        t.n = n[i];
+        t.first = (int)blocks;
+        t.w = w[i];
+        t.grad = grad[i];
+        t.m = m[i];
+        t.v = v[i];
+        t.wb = (__nv_bfloat16 *)wb[i];
+        blocks += blocks_for(n[i], 256);
+    }
+    if (blocks == 0) return PS_OK;
     const float c1 = 1.0f - powf(beta1, (float)step), c2 = 1.0f - powf(beta2, (float)step);
-    adam_kernel<<<blocks_for(n, 256), 256, 0, (cudaStream_t)stream>>>(n, w, grad, m, v, lr, beta1, beta2, eps, c1,
-                                                                       c2, (__nv_bfloat16 *)wb);
+    adam_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(a, lr, beta1, beta2, eps, c1, c2);
     SC_CUDA(cudaGetLastError());
     return PS_OK;
+}
+
+extern "C" ps_status ps_mlp_forward(int32_t n_layers, const int32_t *sizes, int32_t rows, const void *const *w,
+                                    const float *const *bias, void *const *h, float *const *hf, void *stream)
+{
+    if (n_layers < 1 || !sizes || rows < 0 || !w || !bias || !h || !hf)
+        return psb_fail(PS_ERR_ARG, "ps_mlp_forward: bad arguments");
+    if (rows == 0) return PS_OK;
+    for (int l = 0; l < n_layers; ++l) {
+        const int k = sizes[l], n = sizes[l + 1];
+        const bool last = l == n_layers - 1;
+        if (k < 1 || n < 1 || !w[l] || !h[l] || (!last && !h[l + 1]) || (last && !hf[l]))
+            return psb_fail(PS_ERR_ARG, "ps_mlp_forward: bad layer");
+        SC_CUDA(launch_gemm(make_gemm(rows, n, k, h[l], k, 1, w[l], 1, k, hf[l], n, bias[l], last ? 0 : 1,
+                                      last ? nullptr : h[l + 1], n),
+                            nullptr, (cudaStream_t)stream));
+    }
+    return PS_OK;
+}
+
+extern "C" ps_status ps_mlp_backward(int32_t n_layers, const int32_t *sizes, int32_t rows, const void *const *w,
+                                     const void *const *h, const float *const *hf, float *const *dz, void *const *dzb,
+                                     float *const *gw, float *const *gb, void *stream)
+{
+    if (n_layers < 1 || !sizes || rows < 0 || !w || !h || !hf || !dz || !dzb || !gw || !gb)
+        return psb_fail(PS_ERR_ARG, "ps_mlp_backward: bad arguments");
+    cudaStream_t s = (cudaStream_t)stream;
+    const int last = n_layers - 1;
+    ColumnSums cs{};
+    unsigned blocks = 0;
+    auto sum_columns = [&]() -> ps_status {
+        if (blocks) column_sum_kernel<<<blocks, 1024, 0, s>>>(cs);
+        SC_CUDA(cudaGetLastError());
+        cs.n = 0;
+        blocks = 0;
+        return PS_OK;
+    };
+    for (int l = last; l >= 0; --l) {
+        const int k = sizes[l], n = sizes[l + 1];
+        if (k < 1 || n < 1 || !w[l] || !gw[l] || !gb[l] || (rows > 0 && (!h[l] || !dz[l] || !dzb[l] || (l > 0 && !hf[l - 1]))))
+            return psb_fail(PS_ERR_ARG, "ps_mlp_backward: bad layer");
+        if (l == last && rows > 0) {
+            const long all = (long)rows * n;
+            to_bf16_kernel<<<blocks_for(all, 256), 256, 0, s>>>(all, dz[l], (__nv_bfloat16 *)dzb[l]);
+            SC_CUDA(cudaGetLastError());
+        }
+        // the weight gradient, and beside it the gradient of the layer below
+        const Gemm grad = make_gemm(n, k, rows, dzb[l], 1, n, h[l], k, 1, gw[l], k, nullptr, 0, nullptr, 0);
+        if (l > 0) {
+            Gemm down = make_gemm(rows, k, n, dzb[l], n, 1, w[l], k, 1, dz[l - 1], k, nullptr, 0, dzb[l - 1], k);
+            down.gate = hf[l - 1];
+            down.ldg = k;
+            SC_CUDA(launch_gemm(down, &grad, s));
+        } else {
+            SC_CUDA(launch_gemm(grad, nullptr, s));
+        }
+        cs.m[cs.n] = {rows, n, (int)blocks, dz[l], gb[l]};
+        cs.n += 1;
+        blocks += blocks_for(n, 32);
+        if (cs.n == 16 && l > 0) {
+            const ps_status st = sum_columns();
+            if (st != PS_OK) return st;
+        }
+    }
+    return sum_columns();
 }
 
 extern "C" ps_status ps_to_bf16(int64_t n, const float *x, void *y, void *stream)
@@ -657,10 +1003,9 @@ extern "C" ps_status ps_screen_rank(int32_t device, int32_t n_points, const doub
         const float *b = d_par + off + (size_t)n * k;
         off += (size_t)n * k + n;
         const bool last = l == n_layers - 1;
-        dim3 grid((n + kGemmTN - 1) / kGemmTN, (n_freq + kGemmTM - 1) / kGemmTM);
-        gemm_bf16_kernel<<<grid, 128>>>(n_freq, n, k, d_h[cur], k, 1, W, 1, k, last ? d_out : nullptr, n, 0, b,
-                                        last ? 0 : 1, last ? nullptr : d_h[1 - cur], n);
-        e = cudaGetLastError();
+        e = launch_gemm(make_gemm(n_freq, n, k, d_h[cur], k, 1, W, 1, k, last ? d_out : nullptr, n, b, last ? 0 : 1,
+                                  last ? nullptr : d_h[1 - cur], n),
+                        nullptr, nullptr);
         cur = 1 - cur;
     }
     if (e == cudaSuccess) e = cudaMemcpy(score, d_out, sizeof(float) * n_freq, cudaMemcpyDeviceToHost);

@@ -107,6 +107,9 @@ _SIGS = {
     "ps_column_sum": (C.c_int, [C.c_int32, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p]),
     "ps_adam_step": (C.c_int, [C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_float, C.c_float,
                                C.c_float, C.c_float, C.c_int32, C.c_void_p, C.c_void_p]),
+    "ps_adam_steps": (C.c_int, [C.c_int32] + [C.c_void_p] * 6 + [C.c_float] * 4 + [C.c_int32, C.c_void_p]),
+    "ps_mlp_forward": (C.c_int, [C.c_int32, C.c_void_p, C.c_int32] + [C.c_void_p] * 5),
+    "ps_mlp_backward": (C.c_int, [C.c_int32, C.c_void_p, C.c_int32] + [C.c_void_p] * 8),
     "ps_to_bf16": (C.c_int, [C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p]),
     "ps_n_coef": (C.c_int32, [C.c_int32, C.c_int32]),
     "ps_measure_fp64_peak": (C.c_int, [C.c_int32, _dp]),

@@ -67,6 +67,10 @@ def _ptr(t):
     return C.c_void_p(t.data_ptr()) if t is not None else None
 
 
+def _ptrs(ts):
+    return (C.c_void_p * len(ts))(*[t.data_ptr() if t is not None else None for t in ts])
+
+
 class Mlp:
     """The screening network on the device: BF16 weights and activations for
     the tensor cores, FP32 master weights, Adam moments and gradients."""
@@ -105,18 +109,19 @@ class Mlp:
         if xb.dim() != 2 or xb.shape[1] != self.sizes[0] or xb.dtype != torch.bfloat16 or not xb.is_contiguous():
             raise ValueError("Mlp.forward: input must be a contiguous [B, %d] bfloat16 tensor" % self.sizes[0])
         B = xb.shape[0]
-        self.hb, self.hf = [xb], [None]
         L = len(self.W)
-        for l in range(L):
-            n, k = self.W[l].shape
-            last = l == L - 1
-            hf = torch.empty((B, n), dtype=torch.float32, device=self.device)
-            hb = None if last else torch.empty((B, n), dtype=torch.bfloat16, device=self.device)
-            native._check(_lib().ps_gemm_bf16(B, n, k, _ptr(self.hb[-1]), k, 1, _ptr(self.Wb[l]), 1, k, _ptr(hf), n,
-                                              0, _ptr(self.b[l]), 0 if last else 1, _ptr(hb), n, self._stream()))
-            self.hf.append(hf)
-            self.hb.append(hb)
+        widths = self.sizes[1:]
+        hf = torch.empty(B * sum(widths), dtype=torch.float32, device=self.device).split([B * n for n in widths])
+        hb = torch.empty(B * sum(widths[:-1]), dtype=torch.bfloat16, device=self.device)
+        hb = hb.split([B * n for n in widths[:-1]]) if L > 1 else ()
+        self.hf = [None] + [t.view(B, n) for t, n in zip(hf, widths)]
+        self.hb = [xb] + [t.view(B, n) for t, n in zip(hb, widths)] + [None]
+        native._check(_lib().ps_mlp_forward(L, self._sizes(), B, _ptrs(self.Wb), _ptrs(self.b), _ptrs(self.hb[:-1]),
+                                            _ptrs(self.hf[1:]), self._stream()))
         return self.hf[-1][:, 0]
+
+    def _sizes(self):
+        return (C.c_int32 * len(self.sizes))(*self.sizes)
 
     def backward(self, dyhat):
         """dyhat: [B] FP32 loss gradient of the predictions.  Returns the
@@ -126,36 +131,27 @@ class Mlp:
         if dyhat.dim() != 1 or B != self.hb[0].shape[0] or dyhat.dtype != torch.float32:
             raise ValueError("Mlp.backward: gradient must be FP32 [B] for the last forward batch")
         L = len(self.W)
-        dz = dyhat.reshape(B, 1).contiguous()
-        dzb = torch.empty((B, 1), dtype=torch.bfloat16, device=self.device)
-        native._check(_lib().ps_to_bf16(B, _ptr(dz), _ptr(dzb), self._stream()))
-        gW, gb = [None] * L, [None] * L
-        for l in range(L - 1, -1, -1):
-            n, k = self.W[l].shape
-            gW[l] = torch.empty((n, k), dtype=torch.float32, device=self.device)
-            gb[l] = torch.empty(n, dtype=torch.float32, device=self.device)
-            native._check(_lib().ps_gemm_bf16(n, k, B, _ptr(dzb), 1, n, _ptr(self.hb[l]), k, 1, _ptr(gW[l]), k, 0,
-                                              None, 0, None, 0, self._stream()))
-            native._check(_lib().ps_column_sum(B, n, _ptr(dz), _ptr(gb[l]), self._stream()))
-            if l > 0:
-                dh = torch.empty((B, k), dtype=torch.float32, device=self.device)
-                native._check(_lib().ps_gemm_bf16(B, k, n, _ptr(dzb), n, 1, _ptr(self.Wb[l]), k, 1, _ptr(dh), k, 0,
-                                                  None, 0, None, 0, self._stream()))
-                dz = torch.empty((B, k), dtype=torch.float32, device=self.device)
-                dzb = torch.empty((B, k), dtype=torch.bfloat16, device=self.device)
-                native._check(_lib().ps_relu_backward(B * k, _ptr(dh), _ptr(self.hf[l]), _ptr(dz), _ptr(dzb),
-                                                      self._stream()))
+        widths = self.sizes[1:]
+        dz = list(torch.empty(B * sum(widths[:-1]), dtype=torch.float32, device=self.device)
+                  .split([B * n for n in widths[:-1]])) if L > 1 else []
+        dz.append(dyhat.reshape(B, 1).contiguous())
+        dzb = torch.empty(B * sum(widths), dtype=torch.bfloat16, device=self.device).split([B * n for n in widths])
+        gW = [torch.empty_like(w) for w in self.W]
+        gb = [torch.empty_like(b) for b in self.b]
+        native._check(_lib().ps_mlp_backward(L, self._sizes(), B, _ptrs(self.Wb), _ptrs(self.hb[:-1]),
+                                             _ptrs(self.hf[1:]), _ptrs(dz), _ptrs(dzb), _ptrs(gW), _ptrs(gb),
+                                             self._stream()))
         return gW, gb
 
     def adam(self, gW, gb, lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8):
         self.steps += 1
-        for l in range(len(self.W)):
-            native._check(_lib().ps_adam_step(self.W[l].numel(), _ptr(self.W[l]), _ptr(gW[l]), _ptr(self.mW[l]),
-                                              _ptr(self.vW[l]), lr, beta1, beta2, eps, self.steps,
-                                              _ptr(self.Wb[l]), self._stream()))
-            native._check(_lib().ps_adam_step(self.b[l].numel(), _ptr(self.b[l]), _ptr(gb[l]), _ptr(self.mb[l]),
-                                              _ptr(self.vb[l]), lr, beta1, beta2, eps, self.steps, None,
-                                              self._stream()))
+        w, g = self.W + self.b, list(gW) + list(gb)
+        m, v, wb = self.mW + self.mb, self.vW + self.vb, self.Wb + [None] * len(self.b)
+        for i in range(0, len(w), 32):  # tensors of one launch
+            k = slice(i, i + 32)
+            n = (C.c_int64 * len(w[k]))(*[t.numel() for t in w[k]])
+            native._check(_lib().ps_adam_steps(len(w[k]), n, _ptrs(w[k]), _ptrs(g[k]), _ptrs(m[k]), _ptrs(v[k]),
+                                               _ptrs(wb[k]), lr, beta1, beta2, eps, self.steps, self._stream()))
 
     def train_step(self, xb, y, lr=1e-3):
         """One Adam step on the mean squared error; returns the loss."""
