@@ -289,22 +289,17 @@ int launch_fit_teams(const DevObject &o, const DevParams &p, const FitItem *item
 
 int launch_eval(const DevObject &o, const DevParams &p, EvalOut ev, double *scratch, void *stream)
 {
-    TeamLaunch l;
+    // the largest team the GPU holds; where one CTA of this layout fits, a pair does
     for (int k = 2; k >= 0; --k) {
         if (max_teams(o, kTeamSizes[k]) < 1) continue;
+        TeamLaunch l;
         const int e = l.prepare(o, 1, kTeamSizes[k], stream);
         if (e) return e;
         return (int)cudaLaunchKernelEx(&l.cfg, l.fn, o, p, (const FitItem *)nullptr, 1, (int *)nullptr,
                                        (FitOut *)nullptr, scratch, (size_t)0, (int *)nullptr, ev, 1,
                                        (const DevObject *)nullptr, (const DevParams *)nullptr);
     }
-    KernelFn fn;
-    size_t smem;
-    const int e = prepare_kernel(o, &fn, &smem);
-    if (e) return e;
-    fn<<<1, kThreads, smem, (cudaStream_t)stream>>>(o, p, nullptr, 1, nullptr, nullptr, scratch, 0, nullptr,
-                                                    ev, 1, nullptr, nullptr);
-    return (int)cudaGetLastError();
+    return (int)cudaErrorLaunchOutOfResources;
 }
 
 }  // namespace psb

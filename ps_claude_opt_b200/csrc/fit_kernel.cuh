@@ -2240,16 +2240,27 @@ __device__ double evaluate(const DevObject &o, const DevParams &p, const Sh &s, 
 // pivot i+1 runs inside the elimination of pivot i, on the values just
 // written.
 //
-// Thread (rsub, csub) owns row slots rsub + 64 r and columns csub + 4 j.  A
+// Thread (rsub, csub) owns row slots rsub + 64 r and columns csub + 4 j, and
+// holds their values in registers; every update is stored to shared memory too,
+// where the pivot row and each row's pivot-column value are read (the loads of
+// the own values were half of the elimination's shared-memory traffic).  A
 // row swap only swaps the logical labels of two slots (kept in registers), so
 // rows never move.  The pivot row is not scaled when it is chosen: every
 // reader forms the scaled value pivot_row[l] * pivinv itself (the same
-// rounding as a stored product), and the row's owners apply the scale when
-// they next touch it, in the following elimination.  ipiv lives in register
-// bit masks, alike in all threads.  The rounding of every stored value equals
-// the serial algorithm's; the inverse is not needed, so already-pivoted
-// columns are left stale.  Returns the reference's error code: 0, 1 (pivot
-// bookkeeping) or 2 (zero pivot).  All threads must call it.
+// rounding as a stored product), and the row's owners apply the scale in the
+// following elimination.  ipiv lives in register bit masks, alike in all
+// threads.  The rounding of every stored value equals the serial algorithm's;
+// the inverse is not needed, so already-pivoted columns are left stale.
+//
+// What bounds it: the serial chain of one pivot -- the warps' search, the
+// barrier, the division, the update -- on one eighth of the lanes' issue slots.
+// So the update keeps its loads, multiplications, stores and comparisons in
+// separate unrolled stretches without a branch, each a set of independent
+// chains: with one branch per column, values read from shared memory, a pivot
+// of 56 columns took 1630 cycles in the update of about 2250, now 1130 of 1950;
+// a solve inside a production fit 127 k -> 103 k cycles.
+// Returns the reference's error code: 0, 1 (pivot bookkeeping) or 2 (zero
+// pivot).  All threads must call it.  red: candidates; ctl: C_GJROW0.
 struct __align__(16) GjCand {
     double v;  // |a| of the warp's best candidate, -1 if it has none
     int key;   // logical row * n + column
@@ -2280,7 +2291,7 @@ __device__ __forceinline__ int gj_argmax(int hi, unsigned lo, int key)
 // kMaxN: the largest n the caller passes (row slots and columns per thread
 // are sized for it).
 template <int kMaxN>
-static __device__ int gauss_jordan(const Sh &s, int n)
+__device__ __forceinline__ int gauss_jordan(double *A, double *b, double *red, int *ctl, int ld, int n)
 {
     constexpr int kSlots = kThreads / 4;
     constexpr int kRowsPer = (kMaxN + kSlots - 1) / kSlots;
@@ -2290,10 +2301,9 @@ static __device__ int gauss_jordan(const Sh &s, int n)
     static_assert(sizeof(GjCand) * 2 * kWarps <= sizeof(double) * kWarps * 4, "candidate buffers in red");
     static_assert(kWarps <= 32 && (kWarps & (kWarps - 1)) == 0, "one lane per warp candidate");
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int ld = s.ld, rsub = tid >> 2, csub = tid & 3;
+    const int rsub = tid >> 2, csub = tid & 3;
     const unsigned ndiv = ((1u << 20) + n - 1) / n;  // key / n == (key * ndiv) >> 20 for key < n * n
-    double *A = s.covar, *b = s.da;
-    GjCand *cand_buf = reinterpret_cast<GjCand *>(s.red);
+    GjCand *cand_buf = reinterpret_cast<GjCand *>(red);
 
     int lab[kRowsPer];
 #pragma unroll
@@ -2301,6 +2311,7 @@ static __device__ int gauss_jordan(const Sh &s, int n)
     unsigned g1a = 0, g1b = 0, g1c = 0;  // columns with ipiv >= 1
     unsigned g2a = 0, g2b = 0, g2c = 0;  // columns with ipiv >= 2
     unsigned c1 = 0, c2 = 0;             // the same for this thread's columns, bit j = column csub + 4 j
+    const unsigned own_cols = (1u << ((n - csub + 3) >> 2)) - 1;  // bit j: column csub + 4 j < n
     int pend = -1;                       // slot of the previous pivot row (scale pending)
     double pend_inv = 1.0;
 
@@ -2321,26 +2332,23 @@ static __device__ int gauss_jordan(const Sh &s, int n)
         return !(gj_mask_bit(g1a, g1b, g1c, L) && !gj_mask_bit(g2a, g2b, g2c, L));
     };
 
+    double v[kRowsPer][kColsPer];  // the thread's values
 #pragma unroll
     for (int r = 0; r < kRowsPer; ++r) {
         const int ll = rsub + kSlots * r;
-        if (ll < n) {
-            const double *row = A + ll * ld;
-            double big = -1.0;
-            int bj = 0;
+        double big = -1.0;
+        int bj = 0;
 #pragma unroll
-            for (int j = 0; j < kColsPer; ++j) {
-                const int l = csub + 4 * j;
-                if (l < n) {
-                    const double t = fabs(row[l]);
-                    if (t >= big) {
-                        big = t;
-                        bj = j;
-                    }
-                }
+        for (int j = 0; j < kColsPer; ++j) {
+            const int l = csub + 4 * j;
+            v[r][j] = ll < n && l < n ? A[ll * ld + l] : 0.0;
+            const double t = fabs(v[r][j]);
+            if (l < n && t >= big) {
+                big = t;
+                bj = j;
             }
-            cand(big, bj, ll, ll);
         }
+        if (ll < n) cand(big, bj, ll, ll);
     }
 
     int err = 0;
@@ -2389,18 +2397,18 @@ static __device__ int gauss_jordan(const Sh &s, int n)
                 const int ll = rsub + kSlots * r;
                 if (ll >= n) continue;
                 if (ll == pend) {
-                    double *row = A + ll * ld;
 #pragma unroll
                     for (int j = 0; j < kColsPer; ++j) {
                         const int l = csub + 4 * j;
-                        if (l < n && !((c1 >> j) & 1u)) row[l] = __dmul_rn(row[l], pend_inv);
+                        v[r][j] = __dmul_rn(v[r][j], pend_inv);
+                        if (l < n) A[ll * ld + l] = v[r][j];
                     }
                     if (csub == 0) b[ll] = __dmul_rn(b[ll], pend_inv);
                 }
-                if (lab[r] == 0 && csub == 0) s.ctl[C_GJROW0] = ll;
+                if (lab[r] == 0 && csub == 0) ctl[C_GJROW0] = ll;
             }
             __syncthreads();
-            P = s.ctl[C_GJROW0];
+            P = ctl[C_GJROW0];
             pend = -1;
         }
         // the swap of rows irow and icol
@@ -2441,13 +2449,27 @@ static __device__ int gauss_jordan(const Sh &s, int n)
         bslot = 0;
         bad = false;
         const double *__restrict__ prow = A + P * ld;
-#pragma unroll 1
+        const unsigned todo = own_cols & ~c1;  // this thread's columns still to pivot
+        // the scaled pivot row, read whole before the first store of an update
+        // (a load behind a store waits for it: the two may alias)
+        double pr[kColsPer];
+#pragma unroll
+        for (int j = 0; j < kColsPer; ++j) pr[j] = 4 * j < n ? prow[csub + 4 * j] : 0.0;
+#pragma unroll
+        for (int j = 0; j < kColsPer; ++j) pr[j] = __dmul_rn(pr[j], pivinv);
+        double cbs[kRowsPer], bls[kRowsPer];
+#pragma unroll
+        for (int r = 0; r < kRowsPer; ++r) {
+            const int ll = min(rsub + kSlots * r, n - 1);
+            cbs[r] = A[ll * ld + icol];
+            bls[r] = b[ll];
+        }
+#pragma unroll
         for (int r = 0; r < kRowsPer; ++r) {
             const int ll = rsub + kSlots * r;
             if (ll >= n) continue;
-            const int L = r == 0 ? lab[0] : lab[kRowsPer - 1];
+            const int L = lab[r];
             const bool open = row_open(L);
-            double *__restrict__ row = A + ll * ld;
             if (open && c2) bad = true;  // a column with ipiv > 1 in an open row
             double big = -1.0;
             int bj = 0;
@@ -2457,7 +2479,7 @@ static __device__ int gauss_jordan(const Sh &s, int n)
                     for (int j = 0; j < kColsPer; ++j) {
                         const int l = csub + 4 * j;
                         if (l < n && !((c1 >> j) & 1u)) {
-                            const double t = fabs(__dmul_rn(row[l], pivinv));
+                            const double t = fabs(__dmul_rn(v[r][j], pivinv));
                             if (t >= big) {
                                 big = t;
                                 bj = j;
@@ -2468,24 +2490,45 @@ static __device__ int gauss_jordan(const Sh &s, int n)
                 }
                 continue;
             }
-            // x * 1.0 == x exactly: rows other than the pending one pass unscaled
-            const double rs = ll == pend ? pend_inv : 1.0;
-            const double cb = __dmul_rn(row[icol], rs);
+            double cb = cbs[r], bl = bls[r];
+            if (ll == pend) {  // the previous pivot row's scale
+                cb = __dmul_rn(cb, pend_inv);
+                bl = __dmul_rn(bl, pend_inv);
+#pragma unroll
+                for (int j = 0; j < kColsPer; ++j) v[r][j] = __dmul_rn(v[r][j], pend_inv);
+            }
+            // done columns (and those past n, in the row's padding) compute on
+            // and are neither stored nor candidates.  Four running maxima, each
+            // the last of equal values, then the last of the four's largest.
+            double *__restrict__ row = A + ll * ld;
+            constexpr int kRun = 4;
+            double best[kRun];
+            int at[kRun];
+#pragma unroll
+            for (int k = 0; k < kRun; ++k) {
+                best[k] = -1.0;
+                at[k] = 0;
+            }
+#pragma unroll
+            for (int j = 0; j < kColsPer; ++j) v[r][j] = __fma_rn(-pr[j], cb, v[r][j]);
+#pragma unroll
+            for (int j = 0; j < kColsPer; ++j)
+                if ((todo >> j) & 1u) row[csub + 4 * j] = v[r][j];
 #pragma unroll
             for (int j = 0; j < kColsPer; ++j) {
-                const int l = csub + 4 * j;
-                if (l < n && !((c1 >> j) & 1u)) {
-                    const double v = __fma_rn(-__dmul_rn(prow[l], pivinv), cb, __dmul_rn(row[l], rs));
-                    row[l] = v;
-                    const double t = fabs(v);
-                    if (t >= big) {
-                        big = t;
-                        bj = j;
-                    }
-                }
+                const double t = (todo >> j) & 1u ? fabs(v[r][j]) : -2.0;
+                const bool take = t >= best[j % kRun];
+                best[j % kRun] = take ? t : best[j % kRun];
+                at[j % kRun] = take ? j : at[j % kRun];
             }
+#pragma unroll
+            for (int k = 0; k < kRun; ++k)
+                if (best[k] > big || (best[k] == big && best[k] >= 0.0 && at[k] > bj)) {
+                    big = best[k];
+                    bj = at[k];
+                }
             if (open) cand(big, bj, L, ll);
-            if (csub == 0) b[ll] = __fma_rn(-bs, cb, __dmul_rn(b[ll], rs));
+            if (csub == 0) b[ll] = __fma_rn(-bs, cb, bl);
         }
         pend = P;
         pend_inv = pivinv;
@@ -2537,10 +2580,18 @@ static __device__ __noinline__ double trial_call(const DevObject &o, const DevPa
     return trial_chisq<MIXED, true>(o, p, s, rows, perm, conw_r);
 }
 
-template <int kMaxN>
+// for mfit <= ma = n_coef + 8 <= NCP + 8 (and < kMaxFit)
+template <int NCP>
+__device__ __forceinline__ int solve(const Sh &s, int n)
+{
+    constexpr int kMaxN = NCP + 8 < kMaxFit ? NCP + 8 : kMaxFit;
+    return gauss_jordan<kMaxN>(s.covar, s.da, s.red, s.ctl, s.ld, n);
+}
+
+template <int NCP>
 static __device__ __noinline__ int solve_call(const Sh &s, int n)
 {
-    return gauss_jordan<kMaxN>(s, n);
+    return solve<NCP>(s, n);
 }
 
 template <int NCP, bool MIXED, bool CL>
@@ -2617,13 +2668,11 @@ __device__ __forceinline__ void fit_one(const DevObject &o, const DevParams &p, 
         if (tid < mfit) s.da[tid] = s.beta[tid];
         __syncthreads();
         tmark(p, s, T_REST);
-        // mfit <= ma = n_coef + 8 <= NCP + 8 (and < kMaxFit)
-        constexpr int kMaxN = NCP + 8 < kMaxFit ? NCP + 8 : kMaxFit;
         int err;
         if constexpr (CL)
-            err = solve_call<kMaxN>(s, mfit);
+            err = solve_call<NCP>(s, mfit);
         else
-            err = gauss_jordan<kMaxN>(s, mfit);
+            err = solve<NCP>(s, mfit);
         tmark(p, s, T_SOLVE);
         if (err == 0 || err == 2) {
             if (tid < mfit) s.atry[s.fidx[tid]] = s.a[s.fidx[tid]] + s.da[tid];
@@ -2764,18 +2813,18 @@ fit_kernel(DevObject obj, DevParams prm, const FitItem *items, int n_items, int 
     }
     __syncthreads();
 
-    if constexpr (!BATCH) {
-        if (mode == 1) {  // one stand-alone evaluation (parity hook)
+    if constexpr (CL) {
+        // one stand-alone evaluation (parity hook); only in the teams' kernel,
+        // which runs them all: a second copy of the evaluation in this one
+        // made its sweep 1 % slower
+        if (mode == 1) {
             const int ma = o.ma, mfit = o.mfit, ld = s.ld;
             double *cstat = rows + (size_t)o.n_points * o.row_stride;
             int *perm = reinterpret_cast<int *>(rows + scratch_perm(o.n_points, o.row_stride, o.n_curves, ma));
             for (int q = tid; q <= ma; q += kThreads) s.a[q] = ev.a[q];
             __syncthreads();
-            double chisq;
-            if constexpr (CL)
-                chisq = evaluate_call<NCP, MIXED>(o, p, s, s.a, false, s.alpha, s.beta, rows, cstat, perm, p.conw_r);
-            else
-                chisq = evaluate<NCP, MIXED, CL>(o, p, s, s.a, false, s.alpha, s.beta, rows, cstat, perm, p.conw_r);
+            const double chisq =
+                evaluate_call<NCP, MIXED>(o, p, s, s.a, false, s.alpha, s.beta, rows, cstat, perm, p.conw_r);
             if (team.rank() != 0) return;
             for (int idx = tid; idx < mfit * mfit; idx += kThreads) {
                 const int j = idx / mfit, k = idx - j * mfit;

@@ -52,20 +52,15 @@ __global__ void __launch_bounds__(psb::kThreads) solve_probe(const double *a, co
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const int ld = psb::fit_ld(n);
-    psb::Sh s{};
     double *covar = reinterpret_cast<double *>(smem);
     double *da = covar + (size_t)n * ld + (n * ld & 1);
     double *red = da + psb::kMaxFit;
     int *ctl = reinterpret_cast<int *>(red + psb::kWarps * 4);
-    s.covar = covar;
-    s.da = da;
-    s.red = red;
-    s.ctl = ctl;
-    s.ld = ld;
     for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) covar[(idx / n) * ld + idx % n] = a[idx];
     for (int j = threadIdx.x; j < n; j += blockDim.x) da[j] = b[j];
     __syncthreads();
-    const int e = n <= 64 ? psb::gauss_jordan<64>(s, n) : psb::gauss_jordan<psb::kMaxFit>(s, n);
+    const int e = n <= 64 ? psb::gauss_jordan<64>(covar, da, red, ctl, ld, n)
+                          : psb::gauss_jordan<psb::kMaxFit>(covar, da, red, ctl, ld, n);
     for (int j = threadIdx.x; j < n; j += blockDim.x) x[j] = da[j];
     if (threadIdx.x == 0) err[0] = e;
 }
