@@ -599,6 +599,207 @@ Gemm make_gemm(int M, int N, int K, const void *A, long sam, long sak, const voi
     return g;
 }
 
+// ---------------------------------------------------------------- network, forward
+
+// All layers of a network in one launch: a CTA takes 16 MB rows through every
+// layer, their activations in shared memory (and in global memory for the
+// backward pass), the weights streaming past in stages of 64 k's that are
+// fetched kFwdStages - 1 ahead, over the layers' borders.  Warp w computes
+// columns 16 w .. 16 w + 15.  Every result is the same chain of k-steps, bias
+// and rounding as the layers' single products, so the bits are theirs.
+//
+// What bounds it: a layer alone is latency (launch, one tile's loads, 16
+// dependent k-steps), 6 to 13 us for 0.1 to 1 us of tensor work; here the loads
+// run ahead of it and what remains is reading the weights once per CTA from L2.
+// 16 warps a CTA, since two a scheduler left the copies' latency bare (8 warps of
+// 32 columns: 37 us instead of 29 at 5000 rows).
+// MB is the smallest that gives each SM one CTA: 1024 rows take 18 us in CTAs of
+// 16, 25 of 32 and 29 of 48; 3000 rows 33 us of 16 (two waves), 25 of 32.
+// Measured (88-256-256-256-1), layer by layer -> here: 1024 rows 34 -> 18 us,
+// 5000 rows 60 -> 29 us, 65536 rows 335 -> 215 us.
+constexpr int kFwdThreads = 512, kFwdWidth = 256, kFwdLayers = 8, kFwdStages = 3, kFwdK = 64, kFwdMaxMB = 4;
+constexpr int kFwdSW = kFwdK + 8, kFwdSA = kFwdWidth + 8;  // padded rows: no ldmatrix conflicts
+static_assert(kFwdThreads / 32 * 16 == kFwdWidth, "16 columns a warp");
+
+struct MlpForward {
+    struct {
+        int k, n;
+        const __nv_bfloat16 *w;  // [n][k]
+        const float *bias;
+        float *hf;               // [rows][n] FP32 results, or null
+        __nv_bfloat16 *hb;       // the same in BF16, or null (the last layer)
+    } l[kFwdLayers];
+    int n_layers, rows;
+    const __nv_bfloat16 *x;
+};
+
+constexpr size_t forward_smem(int mb)
+{
+    return sizeof(__nv_bfloat16) * ((size_t)kFwdStages * kFwdWidth * kFwdSW + 2 * 16 * (size_t)mb * kFwdSA);
+}
+
+__device__ __forceinline__ void copy16_async(void *dst, const void *src, bool ok)
+{
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+
+template <int MB>
+__global__ void __launch_bounds__(kFwdThreads) mlp_forward_kernel(const MlpForward net)
+{
+    extern __shared__ __align__(16) __nv_bfloat16 fwd_smem[];
+    __nv_bfloat16 *const act = fwd_smem + kFwdStages * kFwdWidth * kFwdSW;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int row0 = blockIdx.x * 16 * MB;
+
+    // the next stage of weights: rows n, columns k0 .. k0 + 63 of its layer,
+    // zeros outside; a thread copies 16 bytes of every kRowStep-th row
+    constexpr int kRowStep = kFwdThreads / (kFwdK / 8);
+    const int pn = tid / (kFwdK / 8), pc = tid % (kFwdK / 8) * 8;
+    int pl = 0, pk = 0, pstage = 0, lk = net.l[0].k, ln = net.l[0].n;
+    const __nv_bfloat16 *lw = net.l[0].w, *src = lw + (size_t)pn * lk + pc;
+    auto prefetch = [&] {
+        if (pl < net.n_layers) {
+            __nv_bfloat16 *dst = fwd_smem + (pstage * kFwdWidth + pn) * kFwdSW + pc;
+            const bool k_in = pk + pc < lk;
+            const size_t step = (size_t)kRowStep * lk;
+#pragma unroll
+            for (int u = 0; u < kFwdWidth / kRowStep; ++u) {
+                const bool ok = k_in && pn + u * kRowStep < ln;
+                if (u * kRowStep < ln) copy16_async(dst + u * kRowStep * kFwdSW, ok ? src + u * step : lw, ok);
+            }
+            pstage = pstage + 1 == kFwdStages ? 0 : pstage + 1;
+            pk += kFwdK;
+            src += kFwdK;
+            if (pk >= lk) {
+                pk = 0;
+                if (++pl < net.n_layers) {
+                    lk = net.l[pl].k;
+                    ln = net.l[pl].n;
+                    lw = net.l[pl].w;
+                    src = lw + (size_t)pn * lk + pc;
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // the input rows, zeros outside
+    {
+        const int k = net.l[0].k, chunks = ((k + 15) & ~15) / 8;
+        for (int i = tid; i < 16 * MB * chunks; i += kFwdThreads) {
+            const int r = i / chunks, c = i % chunks * 8;
+            const bool ok = row0 + r < net.rows && c < k;
+            copy16_async(act + r * kFwdSA + c, ok ? net.x + (size_t)(row0 + r) * k + c : net.x, ok);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kFwdStages - 1; ++i) prefetch();  // the first group holds the input too
+
+    int stage = 0;
+    for (int l = 0; l < net.n_layers; ++l) {
+        const auto &y = net.l[l];
+        const int K = y.k, N = y.n;
+        const __nv_bfloat16 *in = act + (l & 1) * 16 * MB * kFwdSA;
+        const bool active = 16 * warp < N;
+        float acc[MB][2][4];
+#pragma unroll
+        for (int m = 0; m < MB; ++m)
+#pragma unroll
+            for (int n = 0; n < 2; ++n) acc[m][n][0] = acc[m][n][1] = acc[m][n][2] = acc[m][n][3] = 0.0f;
+        for (int k0 = 0; k0 < K; k0 += kFwdK) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kFwdStages - 2) : "memory");
+            __syncthreads();  // this stage has landed, the stage before and the last layer's rows are done
+            prefetch();
+            const int j = lane >> 3, r = lane & 7;
+            const __nv_bfloat16 *wb = fwd_smem + (stage * kFwdWidth + 16 * warp + (j >> 1) * 8 + r) * kFwdSW + (j & 1) * 8;
+            const __nv_bfloat16 *ab = in + ((j & 1) * 8 + r) * kFwdSA + k0 + (j >> 1) * 8;
+            stage = stage + 1 == kFwdStages ? 0 : stage + 1;
+            if (!active) continue;
+            // two k-steps' fragments, then their MMAs
+            uint32_t a[2][MB][4], b[2][4];
+#pragma unroll
+            for (int kk = 0; kk < kFwdK; kk += 32) {
+                if (k0 + kk >= K) break;
+                const bool both = k0 + kk + 16 < K;
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    if (q && !both) break;
+                    ldmatrix4(b[q], wb + kk + 16 * q, false);
+#pragma unroll
+                    for (int m = 0; m < MB; ++m) ldmatrix4(a[q][m], ab + 16 * m * kFwdSA + kk + 16 * q, false);
+                }
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    if (q && !both) break;
+#pragma unroll
+                    for (int m = 0; m < MB; ++m)
+#pragma unroll
+                        for (int n = 0; n < 2; ++n) mma_bf16(acc[m][n], a[q][m], b[q][2 * n], b[q][2 * n + 1]);
+                }
+            }
+        }
+        if (!active) continue;
+        const bool last = l == net.n_layers - 1;
+        __nv_bfloat16 *out = act + ((l + 1) & 1) * 16 * MB * kFwdSA;
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            const int c = 16 * warp + 8 * n + 2 * (lane & 3);
+            const bool in0 = c < N, in1 = c + 1 < N, pair = in1 && !(N & 1);
+            const float b0 = y.bias && in0 ? y.bias[c] : 0.0f, b1 = y.bias && in1 ? y.bias[c + 1] : 0.0f;
+#pragma unroll
+            for (int m = 0; m < MB; ++m)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int r = 16 * m + 8 * h + (lane >> 2);
+                    float v0 = 0.0f + acc[m][n][2 * h], v1 = 0.0f + acc[m][n][2 * h + 1];
+                    if (y.bias) {
+                        v0 += b0;
+                        v1 += b1;
+                    }
+                    if (!last) {
+                        v0 = fmaxf(v0, 0.0f);
+                        v1 = fmaxf(v1, 0.0f);
+                    }
+                    const __nv_bfloat162 hv = __halves2bfloat162(__float2bfloat16(v0), __float2bfloat16(v1));
+                    if (!last) *reinterpret_cast<__nv_bfloat162 *>(out + r * kFwdSA + c) = hv;
+                    if (row0 + r >= net.rows) continue;
+                    const size_t at = (size_t)(row0 + r) * N + c;
+                    if (pair) {
+                        if (y.hf) *reinterpret_cast<float2 *>(y.hf + at) = make_float2(v0, v1);
+                        if (y.hb) *reinterpret_cast<__nv_bfloat162 *>(y.hb + at) = hv;
+                    } else if (in0) {  // an odd width, which only the last layer has
+                        if (y.hf) y.hf[at] = v0;
+                        if (y.hf && in1) y.hf[at + 1] = v1;
+                    }
+                }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+template <int MB>
+cudaError_t launch_forward(const MlpForward &net, cudaStream_t s)
+{
+    const cudaError_t e = cudaFuncSetAttribute(mlp_forward_kernel<MB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)forward_smem(MB));
+    if (e != cudaSuccess) return e;
+    mlp_forward_kernel<MB><<<(net.rows + 16 * MB - 1) / (16 * MB), kFwdThreads, forward_smem(MB), s>>>(net);
+    return cudaGetLastError();
+}
+
+// Whether the one-launch forward pass takes these layers: widths within its
+// tile, weights and input readable in 16-byte pieces, FP32 pairs aligned.  Any
+// other network goes layer by layer.
+bool forward_fits(int n_layers, const int32_t *sizes, const void *const *w, void *const *h, float *const *hf)
+{
+    if (n_layers > kFwdLayers) return false;
+    for (int l = 0; l < n_layers; ++l) {
+        const uintptr_t ptrs = (uintptr_t)w[l] | (uintptr_t)h[l];
+        if (sizes[l] > kFwdWidth || sizes[l + 1] > kFwdWidth || sizes[l] % 8 || ptrs % 16 || (uintptr_t)hf[l] % 8) return false;
+    }
+    return true;
+}
+
 // dZ = dH * (Z > 0), as BF16 (the next backward GEMM's operand) and FP32.
 __global__ void relu_backward_kernel(long n, const float *dh, const float *z, float *dz, __nv_bfloat16 *dzb)
 {
@@ -873,10 +1074,29 @@ extern "C" ps_status ps_mlp_forward(int32_t n_layers, const int32_t *sizes, int3
         return psb_fail(PS_ERR_ARG, "ps_mlp_forward: bad arguments");
     if (rows == 0) return PS_OK;
     for (int l = 0; l < n_layers; ++l) {
+        const bool last = l == n_layers - 1;
+        if (sizes[l] < 1 || sizes[l + 1] < 1 || !w[l] || !h[l] || (!last && !h[l + 1]) || (last && !hf[l]))
+            return psb_fail(PS_ERR_ARG, "ps_mlp_forward: bad layer");
+    }
+    if (forward_fits(n_layers, sizes, w, h, hf)) {
+        MlpForward net{};
+        net.n_layers = n_layers;
+        net.rows = rows;
+        net.x = (const __nv_bfloat16 *)h[0];
+        for (int l = 0; l < n_layers; ++l)
+            net.l[l] = {sizes[l], sizes[l + 1], (const __nv_bfloat16 *)w[l], bias[l], hf[l],
+                        l == n_layers - 1 ? nullptr : (__nv_bfloat16 *)h[l + 1]};
+        const long blocks = ((long)rows + 15) / 16;
+        const int mb = (int)std::min<long>(kFwdMaxMB, (blocks + 147) / 148);
+        SC_CUDA(mb == 1   ? launch_forward<1>(net, (cudaStream_t)stream)
+                : mb == 2 ? launch_forward<2>(net, (cudaStream_t)stream)
+                : mb == 3 ? launch_forward<3>(net, (cudaStream_t)stream)
+                          : launch_forward<4>(net, (cudaStream_t)stream));
+        return PS_OK;
+    }
+    for (int l = 0; l < n_layers; ++l) {
         const int k = sizes[l], n = sizes[l + 1];
         const bool last = l == n_layers - 1;
-        if (k < 1 || n < 1 || !w[l] || !h[l] || (!last && !h[l + 1]) || (last && !hf[l]))
-            return psb_fail(PS_ERR_ARG, "ps_mlp_forward: bad layer");
         SC_CUDA(launch_gemm(make_gemm(rows, n, k, h[l], k, 1, w[l], 1, k, hf[l], n, bias[l], last ? 0 : 1,
                                       last ? nullptr : h[l + 1], n),
                             nullptr, (cudaStream_t)stream));
