@@ -2258,7 +2258,7 @@ __device__ double evaluate(const DevObject &o, const DevParams &p, const Sh &s, 
 // separate unrolled stretches without a branch, each a set of independent
 // chains: with one branch per column, values read from shared memory, a pivot
 // of 56 columns took 1630 cycles in the update of about 2250, now 1130 of 1950;
-// a solve inside a production fit 127 k -> 103 k cycles.
+// a solve inside a production fit 127 k -> 106 k cycles.
 // Returns the reference's error code: 0, 1 (pivot bookkeeping) or 2 (zero
 // pivot).  All threads must call it.  red: candidates; ctl: C_GJROW0.
 struct __align__(16) GjCand {
