@@ -27,12 +27,14 @@ int padded_ncoef(int n_coef)
 size_t fit_smem_bytes(int n_fac, int mfit, int ncp, int n_curves, int row_stride, int tile_rows, int cstat_smem,
                       int mixed)
 {
-    return carve_bytes(n_fac, mfit, ncp, n_curves, row_stride, tile_rows, cstat_smem, mixed, nullptr, nullptr);
+    return kStaticSmem +
+           carve_bytes(n_fac, mfit, ncp, n_curves, row_stride, tile_rows, cstat_smem, mixed, nullptr, nullptr);
 }
 
-static size_t fit_smem_bytes(const DevObject &o)
+size_t fit_dynamic_smem(const DevObject &o)
 {
-    return fit_smem_bytes(o.n_fac, o.mfit, o.ncp, o.n_curves, o.row_stride, o.tile_rows, o.cstat_smem, o.mixed);
+    return carve_bytes(o.n_fac, o.mfit, o.ncp, o.n_curves, o.row_stride, o.tile_rows, o.cstat_smem, o.mixed, nullptr,
+                       nullptr);
 }
 
 int chunk_facets_of(int ncp) { return chunk_facets(ncp); }
@@ -130,7 +132,7 @@ static int prepare_kernel(const DevObject &o, KernelFn *fn, size_t *smem)
 {
     *fn = kernel_for(o.ncp, o.mixed);
     if (!*fn) return (int)cudaErrorInvalidValue;
-    *smem = fit_smem_bytes(o.n_fac, o.mfit, o.ncp, o.n_curves, o.row_stride, o.tile_rows, o.cstat_smem, o.mixed);
+    *smem = fit_dynamic_smem(o);
     cudaError_t e = cudaFuncSetAttribute(*fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem);
     return (int)e;
 }
@@ -162,16 +164,14 @@ int prepare_batch_kernel(const DevObject &env)
 {
     KernelFn fn = batch_kernel_for(env.ncp);
     if (!fn || env.mixed) return (int)cudaErrorInvalidValue;
-    const size_t smem = fit_smem_bytes(env.n_fac, env.mfit, env.ncp, env.n_curves, env.row_stride, env.tile_rows,
-                                       env.cstat_smem, 0);
+    const size_t smem = fit_dynamic_smem(env);
     return (int)cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
 int fit_batch_ctas_per_sm(const DevObject &env)
 {
     if (prepare_batch_kernel(env) != 0) return 0;
-    const size_t smem = fit_smem_bytes(env.n_fac, env.mfit, env.ncp, env.n_curves, env.row_stride, env.tile_rows,
-                                       env.cstat_smem, 0);
+    const size_t smem = fit_dynamic_smem(env);
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_kernel_for(env.ncp), kThreads, smem) != cudaSuccess)
         return 0;
@@ -184,8 +184,7 @@ int launch_fits_batch(const DevObject &env, const DevObject *d_objs, const DevPa
 {
     KernelFn fn = batch_kernel_for(env.ncp);
     if (!fn || env.mixed) return (int)cudaErrorInvalidValue;
-    const size_t smem = fit_smem_bytes(env.n_fac, env.mfit, env.ncp, env.n_curves, env.row_stride, env.tile_rows,
-                                       env.cstat_smem, 0);
+    const size_t smem = fit_dynamic_smem(env);
     DevParams p{};
     EvalOut ev{};
     fn<<<n_ctas, kThreads, smem, (cudaStream_t)stream>>>(env, p, items, n_items, queue, out, scratch,
@@ -202,7 +201,7 @@ struct TeamLaunch {
     {
         fn = team_kernel_for(o.ncp, o.mixed);
         if (!fn) return (int)cudaErrorInvalidValue;
-        const size_t smem = fit_smem_bytes(o);
+        const size_t smem = fit_dynamic_smem(o);
         attr.id = cudaLaunchAttributeClusterDimension;
         attr.val.clusterDim.x = team_size;
         attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
@@ -221,9 +220,9 @@ static int max_teams(const DevObject &o, int team_size)
 {
     TeamLaunch l;
     int n = 0;
-    if (l.prepare(o, 1, team_size, nullptr) != 0) return 0;
-    if (cudaOccupancyMaxActiveClusters(&n, l.fn, &l.cfg) != cudaSuccess) {
-        cudaGetLastError();
+    if (l.prepare(o, 1, team_size, nullptr) != 0 ||
+        cudaOccupancyMaxActiveClusters(&n, l.fn, &l.cfg) != cudaSuccess) {
+        cudaGetLastError();  // not the next launch's
         return 0;
     }
     return n;
@@ -289,7 +288,8 @@ int launch_fit_teams(const DevObject &o, const DevParams &p, const FitItem *item
 
 int launch_eval(const DevObject &o, const DevParams &p, EvalOut ev, double *scratch, void *stream)
 {
-    // the largest team the GPU holds; where one CTA of this layout fits, a pair does
+    // the largest team the GPU holds; where one CTA of a layout fits, a pair does:
+    // the layout was chosen with the teams' static shared memory counted in
     for (int k = 2; k >= 0; --k) {
         if (max_teams(o, kTeamSizes[k]) < 1) continue;
         TeamLaunch l;

@@ -78,9 +78,16 @@ enum StatusBits : int {
     kStatusTimeout = 4,   // a bounded wait on a bulk copy gave up
 };
 
-// Bytes of dynamic shared memory one fit CTA needs.
+// Shared memory a fit CTA may hold statically beside its layout: the one-CTA
+// kernel has none, the teams' kernel 736 bytes (TeamShared), the batch kernel
+// the item's object and constants.
+constexpr size_t kStaticSmem = 1120;
+// Bytes of shared memory one fit CTA needs: the layout, and kStaticSmem.  A
+// layout is chosen by this, so that each kernel can run it; the launches ask
+// for the layout alone (fit_dynamic_smem).
 size_t fit_smem_bytes(int n_fac, int mfit, int ncp, int n_curves, int row_stride, int tile_rows, int cstat_smem,
                       int mixed);
+size_t fit_dynamic_smem(const DevObject &o);
 // Largest padded coefficient count the mixed-precision sweep is built for.
 constexpr int kMaxMixedNcp = 64;
 // Facets per basis chunk of the facet sweep for a padded coefficient count.

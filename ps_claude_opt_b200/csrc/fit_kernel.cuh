@@ -90,11 +90,6 @@ struct Sh {
     unsigned long long *mbar;  // [kStages] completion barriers of the chunk copies
     long long *tclk;  // [T_NPHASE + 1] phase clocks, last slot = previous mark
     int *hist;        // [2][kSortCells] point-sort histogram and offsets
-    double *rdy;      // [kTile] per-row residual y - ymod
-    double *rw;       // [kTile] per-row weight sigr2 * weight
-    double *rcoef;    // [kTile] per-row renormalisation coefficient (relative curves)
-    double *rsub;     // [kTile] per-row ymod * rave (relative curves)
-    int *rcur;        // [kTile] per-row curve index if relative, else -1
     double *red;      // [kWarps * 4]
     double *inv;      // [40] per-evaluation invariants
     double *scal;     // [S_NSCAL]
@@ -236,6 +231,7 @@ __host__ __device__ inline size_t scratch_perm(int n_points, int row_stride, int
     return scratch_gpart(n_points, row_stride, n_curves, ma) + (size_t)kWarps * 36 * 64;
 }
 
+// Dynamic shared memory of one CTA, carved at base.
 __host__ __device__ inline size_t carve_bytes(int n_fac, int mfit, int ncp, int n_curves, int rs, int tr,
                                               int cstat_smem, int mixed, Sh *s, unsigned char *base)
 {
@@ -262,11 +258,6 @@ __host__ __device__ inline size_t carve_bytes(int n_fac, int mfit, int ncp, int 
     const size_t tiles = 2 * tsz + 2 * rsz + 2 * csz;
     const size_t chunks = (size_t)kStages * sizeof(double) * chunk_facets(ncp) * ncp;
     unsigned char *un = (unsigned char *)take(tiles > chunks ? tiles : chunks);
-    void *rdy = take(sizeof(double) * kTile);
-    void *rw = take(sizeof(double) * kTile);
-    void *rcoef = take(sizeof(double) * kTile);
-    void *rsub = take(sizeof(double) * kTile);
-    void *rcur = take(sizeof(int) * kTile);
     void *red = take(sizeof(double) * kWarps * 4);
     void *inv = take(sizeof(double) * 40);
     void *scal = take(sizeof(double) * S_NSCAL);
@@ -292,8 +283,6 @@ __host__ __device__ inline size_t carve_bytes(int n_fac, int mfit, int ncp, int 
         s->raw = (double *)(un + 2 * tsz);
         s->recb = (double4 *)(un + 2 * tsz + 2 * rsz);
         s->ybuf = (double *)un;
-        s->rdy = (double *)rdy; s->rw = (double *)rw;
-        s->rcoef = (double *)rcoef; s->rsub = (double *)rsub; s->rcur = (int *)rcur;
         s->red = (double *)red; s->inv = (double *)inv; s->scal = (double *)scal;
         s->fidx = (int *)fidx; s->ctl = (int *)ctl;
         s->mbar = (unsigned long long *)mbar; s->tbar = (unsigned long long *)tbar;
@@ -2564,6 +2553,8 @@ struct TeamShared {
     DevParams p;
     Sh s;
 };
+static_assert(sizeof(TeamShared) <= kStaticSmem && sizeof(DevObject) + sizeof(DevParams) <= kStaticSmem,
+              "every layout that is chosen runs as a team and in a batch too");
 
 template <int NCP, bool MIXED>
 static __device__ __noinline__ double evaluate_call(const DevObject &o, const DevParams &p, const Sh &s, const double *a,
