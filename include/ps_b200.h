@@ -199,7 +199,8 @@ ps_status ps_gpu_fit_items_device(ps_gpu *h, int32_t n, const int32_t *d_items,
                                   ps_fit_result *d_out);
 
 /* One function evaluation (the reference's mrqcof) at the 1-based parameter
-   vector a[0..ma]: chi^2, alpha (mfit x mfit row-major) and beta (mfit). */
+   vector a[0..ma]: chi^2, alpha (mfit x mfit row-major) and beta (mfit).
+   After a timeout (PS_DEVSTAT_TIMEOUT) chi^2 is NaN. */
 ps_status ps_gpu_eval(ps_gpu *h, const double *a, double *chisq, double *alpha, double *beta,
                       double *area_sum);
 
@@ -345,6 +346,11 @@ ps_status ps_measure_fp64_peak(int32_t device, double *tflops);
    that nothing completes; *status = PS_DEVSTAT_TIMEOUT when the wait gave up
    (0 if it had completed).  The context stays usable. */
 ps_status ps_probe_wait_timeout(int32_t polls, int32_t *status);
+/* Test hook: the same wait in CTA `rank` of a team (a cluster of 2, 4 or 8
+   CTAs), told to the whole team as the fit kernel does; status[0..size-1]:
+   what each CTA knows after the team's next barrier.  No CTA waits where
+   rank is not in the team. */
+ps_status ps_probe_team_timeout(int32_t polls, int32_t size, int32_t rank, int32_t *status);
 /* Test hook: r[i] = the fit kernel's branch-free reciprocal of d[i], on the
    current device (no reference counterpart). */
 ps_status ps_probe_reciprocal(int32_t n, const double *d, double *r);

@@ -423,7 +423,7 @@ extern "C" ps_status ps_gpu_eval(ps_gpu *h, const double *a, double *chisq, doub
     double *d_area = d_chisq + 1;
     PSB_CUDA(cudaMemcpyAsync(d_a, a, sizeof(double) * (ma + 1), cudaMemcpyHostToDevice, h->stream));
     psb::EvalOut ev{d_alpha, d_beta, d_chisq, d_area, d_a};
-    int e = psb::launch_eval(h->obj, h->prm, ev, h->scratch.ptr, h->stream);
+    int e = psb::launch_eval(h->obj, h->prm, ev, h->scratch.ptr, h->status.ptr, h->stream);
     if (e) return psb_fail_cuda(e, "eval kernel launch");
     std::vector<double> back(need - (ma + 1));
     PSB_CUDA(cudaMemcpyAsync(back.data(), d_alpha, back.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));

@@ -286,7 +286,7 @@ int launch_fit_teams(const DevObject &o, const DevParams &p, const FitItem *item
                                    0, (const DevObject *)nullptr, (const DevParams *)nullptr);
 }
 
-int launch_eval(const DevObject &o, const DevParams &p, EvalOut ev, double *scratch, void *stream)
+int launch_eval(const DevObject &o, const DevParams &p, EvalOut ev, double *scratch, int *status, void *stream)
 {
     // the largest team the GPU holds; where one CTA of a layout fits, a pair does:
     // the layout was chosen with the teams' static shared memory counted in
@@ -296,7 +296,7 @@ int launch_eval(const DevObject &o, const DevParams &p, EvalOut ev, double *scra
         const int e = l.prepare(o, 1, kTeamSizes[k], stream);
         if (e) return e;
         return (int)cudaLaunchKernelEx(&l.cfg, l.fn, o, p, (const FitItem *)nullptr, 1, (int *)nullptr,
-                                       (FitOut *)nullptr, scratch, (size_t)0, (int *)nullptr, ev, 1,
+                                       (FitOut *)nullptr, scratch, (size_t)0, status, ev, 1,
                                        (const DevObject *)nullptr, (const DevParams *)nullptr);
     }
     return (int)cudaErrorLaunchOutOfResources;

@@ -79,7 +79,7 @@ enum StatusBits : int {
 };
 
 // Shared memory a fit CTA may hold statically beside its layout: the one-CTA
-// kernel has none, the teams' kernel 736 bytes (TeamShared), the batch kernel
+// kernel has none, the teams' kernel 704 bytes (TeamShared), the batch kernel
 // the item's object and constants.
 constexpr size_t kStaticSmem = 1120;
 // Bytes of shared memory one fit CTA needs: the layout, and kStaticSmem.  A
@@ -102,9 +102,9 @@ int padded_ncoef(int n_coef);
 int launch_fits(const DevObject &o, const DevParams &p, const FitItem *items, int n_items,
                 int *queue, FitOut *out, double *scratch, size_t scratch_per_cta, int n_ctas,
                 int *status, void *stream);
-// One evaluation at ev.a by a team of CTAs on one scratch slab.
-int launch_eval(const DevObject &o, const DevParams &p, EvalOut ev, double *scratch,
-                void *stream);
+// One evaluation at ev.a by a team of CTAs on one scratch slab; chi^2 is NaN
+// after a timeout.
+int launch_eval(const DevObject &o, const DevParams &p, EvalOut ev, double *scratch, int *status, void *stream);
 // CTAs per SM the fit kernel reaches for this object.
 int fit_ctas_per_sm(const DevObject &o);
 

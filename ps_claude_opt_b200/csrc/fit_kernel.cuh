@@ -188,6 +188,18 @@ struct Team {
         if constexpr (CL) return __ldcg(p);
         return *p;
     }
+    // Sets a flag in shared memory in every CTA of a team; all of them see it
+    // after the next sync().
+    __device__ __forceinline__ void raise(int *flag) const
+    {
+        if constexpr (CL) {
+            for (int r = 0; r < size(); ++r) {
+                uint32_t theirs;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(theirs) : "r"(smem_u32(flag)), "r"(r));
+                asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(theirs), "r"(1) : "memory");
+            }
+        }
+    }
 };
 
 // Charges the cycles since the previous mark to `phase` (thread 0, when the
@@ -1958,6 +1970,12 @@ __device__ double evaluate(const DevObject &o, const DevParams &p, const Sh &s, 
     // the tile phase of one CTA reads the rows back through the bulk-copy
     // (async) proxy
     if constexpr (!CL) asm volatile("fence.proxy.async.global;" ::: "memory");
+    // A team whose CTAs did not all get their copies must leave the fit: rows
+    // are missing, a late copy may yet land where a CTA keeps its own residuals,
+    // and CTAs that decide differently would wait for one another at some
+    // barrier for ever.  After this barrier every CTA has the flag; those of one
+    // iteration depend on no data, so all finish it and leave before the next.
+    if (CL && tid == 0 && s.ctl[C_TIMEOUT]) team.raise(&s.ctl[C_TIMEOUT]);
     team.sync();
     tmark(p, s, T_SWEEP);
 
@@ -2626,6 +2644,7 @@ __device__ __forceinline__ void fit_one(const DevObject &o, const DevParams &p, 
             const int niter = s.ctl[C_NITER];
             s.ctl[C_GO] = ((niter < p.n_iter_max) && (s.scal[S_ITERDIFF] > p.iter_diff_max)) ||
                           (niter < p.n_iter_min);
+            if (CL && s.ctl[C_TIMEOUT]) s.ctl[C_GO] = 0;  // in every CTA of the team
         }
         __syncthreads();
         if (!s.ctl[C_GO]) break;
@@ -2816,39 +2835,31 @@ fit_kernel(DevObject obj, DevParams prm, const FitItem *items, int n_items, int 
             __syncthreads();
             const double chisq =
                 evaluate_call<NCP, MIXED>(o, p, s, s.a, false, s.alpha, s.beta, rows, cstat, perm, p.conw_r);
-            if (team.rank() != 0) return;
-            for (int idx = tid; idx < mfit * mfit; idx += kThreads) {
+            const bool first = team.rank() == 0;
+            for (int idx = tid; first && idx < mfit * mfit; idx += kThreads) {
                 const int j = idx / mfit, k = idx - j * mfit;
                 ev.alpha[idx] = s.alpha[j * ld + k];
             }
-            if (tid < mfit) ev.beta[tid] = s.beta[tid];
-            if (tid == 0) {
-                ev.chisq[0] = chisq;
+            if (first && tid < mfit) ev.beta[tid] = s.beta[tid];
+            if (first && tid == 0) {
+                ev.chisq[0] = s.ctl[C_TIMEOUT] ? nan("") : chisq;
                 ev.area[0] = s.scal[S_AREA];
+                if (s.ctl[C_TIMEOUT]) atomicOr(status, kStatusTimeout);
             }
-            return;
         }
     }
 
     int cur = -1;  // batch: the object whose tables are loaded
-    for (;;) {
+    while (!CL || mode != 1) {
         int item;
         if constexpr (CL) {
             // the team's first CTA takes the next item and hands it on through
-            // the slab; all stop once any of them met a timeout
+            // the slab; after a timeout, which all of them know of, they stop
             int *hand = reinterpret_cast<int *>(rows);
             team.sync();  // the previous fit's slab is free
-            if (tid == 0 && team.rank() == 0) {
-                hand[0] = atomicAdd(queue, 1);
-                hand[1] = 0;
-            }
+            if (tid == 0 && team.rank() == 0) hand[0] = s.ctl[C_TIMEOUT] ? INT_MAX : atomicAdd(queue, 1);
             team.sync();
-            if (tid == 0 && s.ctl[C_TIMEOUT]) {
-                atomicOr(&hand[1], 1);
-                atomicOr(status, kStatusTimeout);
-            }
-            team.sync();
-            item = team.load(&hand[1]) ? n_items : team.load(&hand[0]);
+            item = team.load(&hand[0]);
             team.sync();
         } else {
             if (tid == 0) s.ctl[C_ITEM] = atomicAdd(queue, 1);

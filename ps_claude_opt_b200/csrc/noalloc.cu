@@ -319,7 +319,11 @@ extern "C" ps_status ps_fit_items_noalloc(
     else
         e = psb::launch_fits(o, p, d_items, n, ctl, d_out, scratch, per_slab, pl.main_ctas, ctl + 1, s);
     if (e) return psb_fail_cuda(e, "ps_fit_items_noalloc: fit kernel launch");
+    int flags = 0;
     NA_CUDA(cudaMemcpyAsync(out, arena + o_out, (size_t)n * sizeof(ps_fit_result), cudaMemcpyDeviceToHost, s));
+    NA_CUDA(cudaMemcpyAsync(&flags, arena + o_ctl + sizeof(int), sizeof(int), cudaMemcpyDeviceToHost, s));
     NA_CUDA(cudaStreamSynchronize(s));
+    // CTAs that met a timeout took no further items: some results may not be this call's
+    if (flags & psb::kStatusTimeout) return psb_fail(PS_ERR_CUDA, "ps_fit_items_noalloc: a bulk copy never completed");
     return PS_OK;
 }

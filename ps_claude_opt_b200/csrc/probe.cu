@@ -45,6 +45,23 @@ __global__ void wait_probe(unsigned limit, int *status)
     if (threadIdx.x == 0) status[0] = psb::mbar_wait(&bar, 0, limit) ? 0 : psb::kStatusTimeout;
 }
 
+// The same wait in one CTA of a team, told to all of them as the facet sweep
+// does: status[r] is what CTA r knows after the team's barrier.
+__global__ void team_wait_probe(unsigned limit, int rank, int *status)
+{
+    __shared__ unsigned long long bar;
+    __shared__ int flag;
+    const psb::Team<true> team;
+    if (threadIdx.x == 0) {
+        psb::mbar_init(&bar, 1);
+        flag = 0;
+    }
+    team.sync();
+    if (threadIdx.x == 0 && team.rank() == rank && !psb::mbar_wait(&bar, 0, limit)) team.raise(&flag);
+    team.sync();
+    if (threadIdx.x == 0) status[team.rank()] = flag ? psb::kStatusTimeout : 0;
+}
+
 // The fit kernel's damped solve on one n x n system (one CTA, the kernel's
 // shared-memory layout for covar, da, red and ctl).
 __global__ void __launch_bounds__(psb::kThreads) solve_probe(const double *a, const double *b, int n, double *x,
@@ -111,6 +128,29 @@ extern "C" ps_status ps_probe_wait_timeout(int32_t polls, int32_t *status)
     if (e == cudaSuccess) e = cudaMemcpy(status, d, sizeof(int), cudaMemcpyDeviceToHost);
     cudaFree(d);
     if (e != cudaSuccess) return psb_fail_cuda(e, "ps_probe_wait_timeout");
+    return PS_OK;
+}
+
+extern "C" ps_status ps_probe_team_timeout(int32_t polls, int32_t size, int32_t rank, int32_t *status)
+{
+    if (polls < 1 || (size != 2 && size != 4 && size != 8) || !status)
+        return psb_fail(PS_ERR_ARG, "ps_probe_team_timeout: bad arguments");
+    int *d = nullptr;
+    cudaError_t e = cudaMalloc(&d, size * sizeof(int));
+    if (e != cudaSuccess) return psb_fail_cuda(e, "ps_probe_team_timeout");
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = size;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(size);
+    cfg.blockDim = dim3(32);
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, team_wait_probe, (unsigned)polls, (int)rank, d);
+    if (e == cudaSuccess) e = cudaMemcpy(status, d, size * sizeof(int), cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    if (e != cudaSuccess) return psb_fail_cuda(e, "ps_probe_team_timeout");
     return PS_OK;
 }
 
