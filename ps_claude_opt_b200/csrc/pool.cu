@@ -1,11 +1,13 @@
-// pool.cu -- short-lived device buffers of the screening entry points.
+// pool.cu -- short-lived device buffers of the screening features.
 //
-// cudaMalloc and cudaFree cost more than those calls' kernels, so buffers come
+// cudaMalloc and cudaFree cost more than that call's kernel, so its buffer comes
 // from a stream-ordered pool of the library's own, one per device.  It keeps
 // at most kKept bytes between calls; what it keeps unused the driver takes
 // back when another allocation of the process runs short of memory.  A buffer
 // is used and freed in the order of one stream, so threads and streams share
-// the pool safely.
+// the pool safely.  A pool belongs to the context it was made in: after a
+// cudaDeviceReset the device has another context, and gets another pool.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -17,14 +19,39 @@ namespace {
 constexpr int kMaxDevices = 64;
 constexpr unsigned long long kKept = 32ull << 20;
 
-std::mutex g_mu;
-cudaMemPool_t g_pool[kMaxDevices];
+struct Pool {
+    cudaMemPool_t pool = nullptr;
+    unsigned long long context = 0;
+};
 
+std::mutex g_mu;
+Pool g_pool[kMaxDevices];
+
+// Id of the current device's context: no two contexts of a process have the
+// same, unlike their addresses.
+cudaError_t context_id(unsigned long long *id)
+{
+    using Fn = CUresult (*)(CUcontext, unsigned long long *);
+    static const Fn fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return (Fn)p;
+    }();
+    return fn && fn(nullptr, id) == CUDA_SUCCESS ? cudaSuccess : cudaErrorDeviceUninitialized;
+}
+
+// The current device's pool.
 cudaError_t pool_of(int device, cudaMemPool_t *pool)
 {
     if (device < 0 || device >= kMaxDevices) return cudaErrorInvalidDevice;
+    unsigned long long context = 0;
+    const cudaError_t ce = context_id(&context);
+    if (ce != cudaSuccess) return ce;
     std::lock_guard<std::mutex> lk(g_mu);
-    if (!g_pool[device]) {
+    if (g_pool[device].context != context) {  // none yet, or of a context that is gone
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
@@ -38,9 +65,9 @@ cudaError_t pool_of(int device, cudaMemPool_t *pool)
             cudaMemPoolDestroy(p);
             return e;
         }
-        g_pool[device] = p;
+        g_pool[device] = {p, context};
     }
-    *pool = g_pool[device];
+    *pool = g_pool[device].pool;
     return cudaSuccess;
 }
 
