@@ -228,7 +228,9 @@ ps_status ps_gpu_set_precision(ps_gpu *h, int32_t precision);
    J^T W J tiles (other), pseudo-points, Gauss-Jordan, the rest, the trial
    steps' brightness sweep, tile staging, tile rank-k updates, then the number
    of full evaluations (at the start and after each accepted step) -- and the
-   counters restart; enable = 0 switches them off. */
+   counters restart; enable = 0 switches them off.  A team's fit counts the
+   cycles of its first CTA, and a team's whole J^T W J update (pseudo-points
+   and barriers with it) as rank-k updates. */
 ps_status ps_gpu_phase_clocks(ps_gpu *h, int32_t enable, int64_t *out);
 /* The CUDA stream all work of the handle runs on (a cudaStream_t). */
 void *ps_gpu_stream(ps_gpu *h);

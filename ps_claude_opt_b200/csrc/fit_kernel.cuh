@@ -2029,6 +2029,7 @@ __device__ double evaluate(const DevObject &o, const DevParams &p, const Sh &s, 
         else
             normal_matrix_team<2>(o, s, rows, cstat, dst, dvec, gpart, conw_r);
         tmark(p, s, T_TSYRK);
+        if (p.phase_cycles && tid == 0 && team.rank() == 0) atomicAdd(&p.phase_cycles[T_NPHASE], 1ull);
         return s.scal[S_TRIAL];
     }
 
