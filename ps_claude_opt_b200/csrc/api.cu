@@ -332,17 +332,32 @@ extern "C" ps_status ps_gpu_occupancy(ps_gpu *h, int32_t *ctas_per_sm, int32_t *
 // CTAs, what is left by teams beside them.
 static ps_status enqueue_fits(ps_gpu *h, int n, const psb::FitItem *d_items, psb::FitOut *d_out)
 {
-    const psb::FitPlan pl = psb::plan_fits(h->obj, n, h->ctas_per_sm * h->n_sm, 0, true);
-    PSB_CUDA(h->scratch.ensure(h->scratch_per_cta * (size_t)pl.slabs()));
+    const int resident = h->ctas_per_sm * h->n_sm;
+    psb::FitPlan pl = psb::plan_fits(h->obj, n, resident, 0, true);
+    // A slab for each fit; from a whole wave on for the most teams that could
+    // run beside it too.  With the teams' kernel loaded by any call, a handle that
+    // has run as many fits, or a wave, never allocates again: later calls may be
+    // under capture, and a captured one keeps its slabs.
+    const int slabs = n < resident ? n : resident + resident / 2;
+    cudaError_t se = h->scratch.ensure(h->scratch_per_cta * (size_t)slabs);
+    if (se == cudaErrorMemoryAllocation && n >= resident) {  // no room for the teams: single CTAs alone
+        cudaGetLastError();
+        pl = psb::FitPlan{};
+        pl.main_items = n;
+        pl.main_ctas = std::min(n, resident);
+        se = h->scratch.ensure(h->scratch_per_cta * (size_t)pl.main_ctas);
+    }
+    PSB_CUDA(se);
     PSB_CUDA(cudaMemsetAsync(h->queue.ptr, 0, 2 * sizeof(int), h->stream));
+    psb::load_team_kernel(h->obj);
+    if (n >= resident) {
+        if (!h->side) PSB_CUDA(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
+        if (!h->fork) PSB_CUDA(cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming));
+        if (!h->join) PSB_CUDA(cudaEventCreateWithFlags(&h->join, cudaEventDisableTiming));
+    }
     const bool both = pl.main_items > 0 && pl.team_items > 0;
     cudaStream_t ts = h->stream;
     if (both) {
-        if (!h->side) {
-            PSB_CUDA(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
-            PSB_CUDA(cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming));
-            PSB_CUDA(cudaEventCreateWithFlags(&h->join, cudaEventDisableTiming));
-        }
         ts = h->side;
         PSB_CUDA(cudaEventRecord(h->fork, h->stream));
         PSB_CUDA(cudaStreamWaitEvent(ts, h->fork, 0));

@@ -228,6 +228,12 @@ static int max_teams(const DevObject &o, int team_size)
     return n;
 }
 
+void load_team_kernel(const DevObject &o)
+{
+    TeamLaunch l;
+    if (l.prepare(o, 1, 2, nullptr) != 0) cudaGetLastError();  // the launch itself will say so
+}
+
 constexpr int kTeamSizes[3] = {2, 4, 8};
 // Time of one fit by a team, as a share of its time by one CTA.  Measured, FP64,
 // teams of 2 / 4 / 8: production object 0.73 / 0.42 / 0.27, largest models

@@ -118,6 +118,9 @@ struct FitPlan {
 // resident: CTAs the GPU holds; max_slabs: scratch slabs there is room for (0:
 // any number); mixable: the two kinds may run side by side (two streams).
 FitPlan plan_fits(const DevObject &o, int n, int resident, int max_slabs, bool mixable);
+// Has the teams' kernel for an object loaded (the driver loads kernels when they
+// are first used, into device memory).
+void load_team_kernel(const DevObject &o);
 // Launches one kind of a plan: team_size CTAs per fit, `groups` fits at a time.
 int launch_fit_teams(const DevObject &o, const DevParams &p, const FitItem *items, int n_items, int *queue,
                      FitOut *out, double *scratch, size_t scratch_per_cta, int groups, int team_size, int *status,
