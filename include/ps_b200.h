@@ -327,7 +327,8 @@ ps_status ps_to_bf16(int64_t n, const float *x, void *y, void *stream);
    hf[l] the FP32 output of layer l (hf of a hidden layer may be null).
    Backward: dz[n_layers-1] holds the FP32 gradient of the outputs; dz[l], dzb[l]
    receive each layer's output gradient (FP32, BF16), gw[l], gb[l] the weight
-   and bias gradients; h and hf are the forward pass's. */
+   and bias gradients; h and hf are the forward pass's.  A null array where one
+   is named is refused, also for rows = 0. */
 ps_status ps_mlp_forward(int32_t n_layers, const int32_t *sizes, int32_t rows, const void *const *w,
                          const float *const *bias, void *const *h, float *const *hf, void *stream);
 ps_status ps_mlp_backward(int32_t n_layers, const int32_t *sizes, int32_t rows, const void *const *w,

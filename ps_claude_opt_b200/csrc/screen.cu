@@ -1072,12 +1072,12 @@ extern "C" ps_status ps_mlp_forward(int32_t n_layers, const int32_t *sizes, int3
 {
     if (n_layers < 1 || !sizes || rows < 0 || !w || !bias || !h || !hf)
         return psb_fail(PS_ERR_ARG, "ps_mlp_forward: bad arguments");
-    if (rows == 0) return PS_OK;
     for (int l = 0; l < n_layers; ++l) {
         const bool last = l == n_layers - 1;
         if (sizes[l] < 1 || sizes[l + 1] < 1 || !w[l] || !h[l] || (!last && !h[l + 1]) || (last && !hf[l]))
             return psb_fail(PS_ERR_ARG, "ps_mlp_forward: bad layer");
     }
+    if (rows == 0) return PS_OK;
     if (forward_fits(n_layers, sizes, w, h, hf)) {
         MlpForward net{};
         net.n_layers = n_layers;
@@ -1123,7 +1123,7 @@ extern "C" ps_status ps_mlp_backward(int32_t n_layers, const int32_t *sizes, int
     };
     for (int l = last; l >= 0; --l) {
         const int k = sizes[l], n = sizes[l + 1];
-        if (k < 1 || n < 1 || !w[l] || !gw[l] || !gb[l] || (rows > 0 && (!h[l] || !dz[l] || !dzb[l] || (l > 0 && !hf[l - 1]))))
+        if (k < 1 || n < 1 || !w[l] || !gw[l] || !gb[l] || !h[l] || !dz[l] || !dzb[l] || (l > 0 && !hf[l - 1]))
             return psb_fail(PS_ERR_ARG, "ps_mlp_backward: bad layer");
         if (l == last && rows > 0) {
             const long all = (long)rows * n;
