@@ -354,6 +354,10 @@ ps_status ps_probe_wait_timeout(int32_t polls, int32_t *status);
    what each CTA knows after the team's next barrier.  No CTA waits where
    rank is not in the team. */
 ps_status ps_probe_team_timeout(int32_t polls, int32_t size, int32_t rank, int32_t *status);
+/* Test hook: the wait that ends a kernel after a timeout, on a barrier whose last
+   issued copy is the `uses`-th and of which `done` have landed; *status = 0
+   if it found the last one landed, PS_DEVSTAT_TIMEOUT when it gave up. */
+ps_status ps_probe_last_wait(int32_t polls, int32_t uses, int32_t done, int32_t *status);
 /* Test hook: r[i] = the fit kernel's branch-free reciprocal of d[i], on the
    current device (no reference counterpart). */
 ps_status ps_probe_reciprocal(int32_t n, const double *d, double *r);

@@ -149,6 +149,14 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, uint32_t pari
     return false;
 }
 
+// Waits for the last of the copies that were issued on a barrier, one phase
+// each (at once if there were none: a new barrier's phase before the first
+// counts as complete).
+__device__ __forceinline__ bool mbar_wait_last(unsigned long long *bar, int uses, unsigned limit = kWaitLimit)
+{
+    return mbar_wait(bar, (uint32_t)((uses - 1) & 1), limit);
+}
+
 // The CTAs that work on one fit: one, or a thread-block cluster of 2, 4 or 8
 // that shares the fit's scratch slab in global memory.  Every CTA of a cluster
 // holds the fit's whole state and takes the same decisions; the points of the
@@ -2893,8 +2901,8 @@ fit_kernel(DevObject obj, DevParams prm, const FitItem *items, int n_items, int 
     // after a timeout, give any copy still in flight a bounded chance to land
     // before the CTA's shared memory is released
     if (tid == 0 && s.ctl[C_TIMEOUT]) {
-        for (int b = 0; b < kStages; ++b) mbar_wait(&s.mbar[b], (uint32_t)(s.ctl[C_YUSE + b] & 1));
-        for (int b = 0; b < 2; ++b) mbar_wait(&s.tbar[b], (uint32_t)(s.ctl[C_TUSE + b] & 1));
+        for (int b = 0; b < kStages; ++b) mbar_wait_last(&s.mbar[b], s.ctl[C_YUSE + b]);
+        for (int b = 0; b < 2; ++b) mbar_wait_last(&s.tbar[b], s.ctl[C_TUSE + b]);
     }
 }
 

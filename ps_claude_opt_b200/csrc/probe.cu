@@ -45,6 +45,20 @@ __global__ void wait_probe(unsigned limit, int *status)
     if (threadIdx.x == 0) status[0] = psb::mbar_wait(&bar, 0, limit) ? 0 : psb::kStatusTimeout;
 }
 
+// A barrier of which `done` of `uses` phases are complete: status 0 if the wait
+// that ends a kernel after a timeout finds the last one complete.
+__global__ void last_wait_probe(unsigned limit, int uses, int done, int *status)
+{
+    __shared__ unsigned long long bar;
+    if (threadIdx.x == 0) {
+        psb::mbar_init(&bar, 1);
+        for (int i = 0; i < done; ++i)
+            asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.shared::cta.b64 t, [%0];\n\t}" ::"r"(psb::smem_u32(&bar))
+                         : "memory");
+        status[0] = psb::mbar_wait_last(&bar, uses, limit) ? 0 : psb::kStatusTimeout;
+    }
+}
+
 // The same wait in one CTA of a team, told to all of them as the facet sweep
 // does: status[r] is what CTA r knows after the team's barrier.
 __global__ void team_wait_probe(unsigned limit, int rank, int *status)
@@ -128,6 +142,21 @@ extern "C" ps_status ps_probe_wait_timeout(int32_t polls, int32_t *status)
     if (e == cudaSuccess) e = cudaMemcpy(status, d, sizeof(int), cudaMemcpyDeviceToHost);
     cudaFree(d);
     if (e != cudaSuccess) return psb_fail_cuda(e, "ps_probe_wait_timeout");
+    return PS_OK;
+}
+
+extern "C" ps_status ps_probe_last_wait(int32_t polls, int32_t uses, int32_t done, int32_t *status)
+{
+    if (polls < 1 || done < 0 || done > uses || uses > 1000 || !status)
+        return psb_fail(PS_ERR_ARG, "ps_probe_last_wait: bad arguments");
+    int *d = nullptr;
+    cudaError_t e = cudaMalloc(&d, sizeof(int));
+    if (e != cudaSuccess) return psb_fail_cuda(e, "ps_probe_last_wait");
+    last_wait_probe<<<1, 32>>>((unsigned)polls, uses, done, d);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpy(status, d, sizeof(int), cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    if (e != cudaSuccess) return psb_fail_cuda(e, "ps_probe_last_wait");
     return PS_OK;
 }
 

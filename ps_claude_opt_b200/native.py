@@ -115,6 +115,7 @@ _SIGS = {
     "ps_measure_fp64_peak": (C.c_int, [C.c_int32, _dp]),
     "ps_probe_reciprocal": (C.c_int, [C.c_int32, _dp, _dp]),
     "ps_probe_wait_timeout": (C.c_int, [C.c_int32, _ip]),
+    "ps_probe_last_wait": (C.c_int, [C.c_int32, C.c_int32, C.c_int32, _ip]),
     "ps_probe_team_timeout": (C.c_int, [C.c_int32, C.c_int32, C.c_int32, _ip]),
     "ps_probe_solve": (C.c_int, [C.c_int32, _dp, _dp, _dp, _ip]),
     "ps_last_error": (C.c_char_p, []),
