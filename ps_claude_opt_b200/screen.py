@@ -144,8 +144,9 @@ class Mlp:
         return gW, gb
 
     def adam(self, gW, gb, lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8):
+        L = range(len(self.W))
+        w, g = self.W + self.b, [gW[l] for l in L] + [gb[l] for l in L]
         self.steps += 1
-        w, g = self.W + self.b, list(gW) + list(gb)
         m, v, wb = self.mW + self.mb, self.vW + self.vb, self.Wb + [None] * len(self.b)
         for i in range(0, len(w), 32):  # tensors of one launch
             k = slice(i, i + 32)
