@@ -252,13 +252,14 @@ ps_status ps_gpu_occupancy(ps_gpu *h, int32_t *ctas_per_sm, int32_t *n_sm);
    NULL) does only that -- select the device, load the module, look up the
    array -- so a caller can reserve the 64 MiB at start-up, before its own
    allocator fills the device.  Each call looks up the array's device address
-   with the device current; the first call with work also sets the kernel's
-   shared-memory limit: make it before any stream capture.  Calls share the
+   with the device current; the first call with work also loads the object's
+   two kernels (one CTA a fit, and teams of CTAs) and sets their
+   shared-memory limits: make it before any stream capture.  Calls share the
    array and leave their data in it;
    calls that overlap on the GPU race -- serialise them.  Objects whose tables
    plus one CTA's scratch exceed 64 MiB, or with more than 200 lightcurves,
-   are rejected with PS_ERR_ARG; smaller ones run on as many CTAs as the
-   remaining scratch holds.  stream may be NULL (the legacy default stream);
+   are rejected with PS_ERR_ARG; smaller ones run at most as many fits at a
+   time as the remaining scratch holds, by one CTA each or by teams.  stream may be NULL (the legacy default stream);
    the call returns after the results are in out. */
 ps_status ps_fit_items_noalloc(int32_t device, void *stream, const double *beta_pole,
                                const double *lambda_pole, const double *par, double cl,

@@ -23,16 +23,18 @@
 //     time, before its own allocator grows;
 //   * every call looks up the arena's device address with the device current
 //     (cudaGetSymbolAddress: cheap once the module is loaded, and never stale
-//     after a cudaDeviceReset); the first call with work also sets the fit
-//     kernel's shared-memory limit; make the first call before any stream
-//     capture;
+//     after a cudaDeviceReset); the first call with work also loads the
+//     object's two fit kernels (one CTA a fit, and teams of CTAs; the choice
+//     between them queries both, whatever n is) and sets their shared-memory
+//     limits; make the first call before any stream capture;
 //   * every call reuses the arena and leaves the last call's contents there;
 //     calls that overlap on the GPU (two host threads, or two streams) race
 //     on it -- serialise them;
 //   * an object whose tables plus one CTA's scratch exceed the arena is
-//     rejected with PS_ERR_ARG; otherwise the grid is as many CTAs as the
-//     remaining scratch holds (fewer than the resident maximum for large
-//     objects, so slower than ps_gpu_fit_items, never different).
+//     rejected with PS_ERR_ARG; otherwise the remaining scratch bounds the
+//     fits that run at a time, each by one CTA or by a team (fewer than the
+//     resident maximum for large objects, so slower than ps_gpu_fit_items,
+//     never different: a team's results are one CTA's, bit for bit).
 #include <cuda_runtime.h>
 
 #include <algorithm>
