@@ -36,8 +36,8 @@ FITS_PER_CTA = 10           # fits per resident CTA in one step
 L2_FLUSH_BYTES = 256 << 20  # > 126 MB L2
 # DRAM bytes per fit of the fit kernel on this workload: dram__bytes_read.sum +
 # dram__bytes_write.sum = 5.30 + 6.78 = 12.075 GB over the 148 fits of one
-# ncu capture of `bench.py --profile-case` (profiles/fit_kernel_production_object.md;
-# the derivative-row scratch round trip, which grows with the number of fits,
+# ncu capture of `bench.py --profile-case` (summary under profiles/; the
+# derivative-row scratch round trip, which grows with the number of fits,
 # so a launch's traffic is this times its fits).
 NCU_DRAM_BYTES_PER_FIT = 12.075e9 / 148
 METRIC = ("LM fits/s of the plain FP64 full scan of the production object on 1 B200 (s/object of it and of "
@@ -292,16 +292,20 @@ def result_errors(test, ref, n_points):
             "lines_outside_envelope": c.envelope_violations, "best_line_same": c.best_line_same}
 
 
-def flops_per_fit(obj, niter):
-    """Algorithmic FLOPs of one fit: (niter + 1) evaluations + niter solves,
-    per-point cost F_pt = 150 + 10 Nf + V (60 + 2 nc) + mfit (mfit + 1) +
-    2 mfit + 6 ma [relative], V = 0.45 Nf."""
+def flops_per_fit(obj, niter, full):
+    """FLOPs of one fit as it runs: `full` evaluations with derivatives (at the
+    start and after each accepted step that another follows), niter trials
+    that form chi^2 alone, niter solves.  Per point a full evaluation costs
+    150 + 10 Nf + V (60 + 2 nc) + mfit (mfit + 1) + 2 mfit + 6 ma [relative], a
+    trial 150 + 10 Nf + 15 V, V = 0.45 Nf."""
     nf, nc, mfit, ma = obj.n_fac, obj.n_coef, obj.mfit, obj.ma
     V = 0.45 * nf
     base = 150 + 10 * nf + V * (60 + 2 * nc) + mfit * (mfit + 1) + 2 * mfit
     n_rel = int(sum(l for l, r in zip(obj.curve_len, obj.curve_rel) if r))
-    f_eval = obj.n_points * base + n_rel * 6 * ma + 3 * (2 * nf * nc + 2 * nf) + 2 * nf * nc + nf
-    return (niter + 1) * f_eval + niter * 2.0 * mfit ** 3
+    areas = 2 * nf * nc + nf
+    f_eval = obj.n_points * base + n_rel * 6 * ma + 3 * (2 * nf * nc + 2 * nf) + areas
+    f_trial = obj.n_points * (150 + 10 * nf + 15 * V) + 6 * nf + areas
+    return full * f_eval + niter * (f_trial + 2.0 * mfit ** 3)
 
 
 class ClockSampler:
@@ -428,8 +432,11 @@ def profile_case(mixed=False):
         for _ in range(2):
             res, niter, _ = eng.fit_items(nf, pl)
         assert np.all(np.isfinite(res[:, 2]))
-        print("profile case: %d fits, mean iterations %.1f, flops/launch %.4g" %
-              (n, niter.mean(), flops_per_fit(obj, niter.mean()) * n))
+        eng.phase_clocks(True)
+        eng.fit_items(nf, pl)
+        full = eng.phase_clocks(False)["evals"] / n
+        print("profile case: %d fits, mean iterations %.1f, full evaluations %.1f, flops/launch %.4g" %
+              (n, niter.mean(), full, flops_per_fit(obj, niter.mean(), full) * n))
 
 
 RESULT_DTYPE = np.dtype([("dev", "f8"), ("dark", "f8"), ("per", "f8"), ("la", "f8"), ("be", "f8"),
@@ -557,7 +564,13 @@ def main():
         dist.all_reduce(t, op=dist.ReduceOp.MAX)
         total_ms = float(t.item())
     value = n_fits * args.steps * world / (total_ms / 1000.0)
-    fl = flops_per_fit(obj, niter) * n_fits
+    # full evaluations of the last step's fits, from one more launch of them (not timed)
+    eng.phase_clocks(True)
+    with torch.cuda.stream(stream):
+        run_step(steps_total - 1)
+    torch.cuda.synchronize()
+    full = eng.phase_clocks(False)["evals"] / n_fits
+    fl = flops_per_fit(obj, niter, full) * n_fits
     achieved = fl / (np.mean(ms) / 1000.0) / 1e12
 
     # end to end through the C ABI with host buffers: object upload, items,
@@ -619,7 +632,9 @@ def main():
                          "traffic_source": "ncu capture of the profile case (148 fits), scaled by fits per launch",
                          "peak_source": "measured FP64 FMA probe (ps_measure_fp64_peak) on this GPU; "
                                         "MEASURED_PEAKS.json has no FP64 figure",
-                         "flops_per_launch": fl, "mean_niter": niter},
+                         "flops_per_launch": fl, "mean_niter": niter, "mean_full_evaluations": full,
+                         "flops_counted": "work that runs: a trial step forms chi^2 alone, a full evaluation "
+                                          "follows an accepted step"},
             "clocks": clk,
             "e2e": {"value": e2e_value, "unit": "fits/s", "h2d_bytes_per_step": int(h2d),
                     "d2h_bytes_per_step": int(d2h), "ms_per_step": float(np.mean(e2e_ms)),
