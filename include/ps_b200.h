@@ -259,8 +259,9 @@ ps_status ps_gpu_occupancy(ps_gpu *h, int32_t *ctas_per_sm, int32_t *n_sm);
    calls that overlap on the GPU race -- serialise them.  Objects whose tables
    plus one CTA's scratch exceed 64 MiB, or with more than 200 lightcurves,
    are rejected with PS_ERR_ARG; smaller ones run at most as many fits at a
-   time as the remaining scratch holds, by one CTA each or by teams.  stream may be NULL (the legacy default stream);
-   the call returns after the results are in out. */
+   time as the remaining scratch holds, by one CTA each or by teams.  stream
+   may be NULL (the legacy default stream); the call returns after the results
+   are in out. */
 ps_status ps_fit_items_noalloc(int32_t device, void *stream, const double *beta_pole,
                                const double *lambda_pole, const double *par, double cl,
                                double alamda_start, double alamda_incr, double alamda_incrr,

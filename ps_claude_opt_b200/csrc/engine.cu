@@ -252,10 +252,11 @@ FitPlan plan_fits(const DevObject &o, int n, int resident, int max_slabs, bool m
     pl.main_ctas = std::min(n, wave);
     // with nothing but whole waves, or a last wave too full to split, single
     // CTAs are best; without a second stream all fits go one way.  A wave of
-    // single CTAs takes 1, so teams must make the rest cheaper: with 148 SMs
-    // teams of 8 up to 18 fits (10 production fits: 57.6 -> 15.9 ms), of 4 up to
-    // about 37 (30 fits: 24.5 ms), of 2 up to 74 (70 fits: 42.5 ms), single CTAs
-    // above (140 fits: 58 ms)
+    // single CTAs takes 1, so teams must make the rest cheaper.  B200's 148 SMs
+    // hold 15 teams of 8, 33 of 4 or 74 of 2 at a time, so production fits go by
+    // teams of 8 up to 15 (10 fits: 56.3 -> 15.4 ms), of 4 up to 33 (30 fits: 23.8
+    // ms), of 2 up to 74 (70 fits: 41.7 ms), and by single CTAs above (140 fits:
+    // 56.3 ms)
     const int items = mixable ? rest : n;
     if (items == 0) return pl;
     double best = mixable ? 1.0 : (n + wave - 1) / wave;

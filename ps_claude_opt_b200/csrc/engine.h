@@ -3,7 +3,7 @@
 // One object's constant tables live in HBM once; every CTA of the persistent
 // fit kernel reads them through L1/L2.  Per-fit state lives in shared memory
 // (facet areas, the two LM matrices, parameters); the per-point derivative
-// rows of one evaluation go to a per-CTA scratch slab in HBM/L2.
+// rows of one evaluation go to a scratch slab per fit in flight in HBM/L2.
 #pragma once
 #include <cstddef>
 #include <cstdint>
@@ -79,7 +79,7 @@ enum StatusBits : int {
 };
 
 // Shared memory a fit CTA may hold statically beside its layout: the one-CTA
-// kernel has none, the teams' kernel 704 bytes (TeamShared), the batch kernel
+// kernel has none, the teams' kernel about 700 bytes (TeamShared), the batch kernel
 // the item's object and constants.
 constexpr size_t kStaticSmem = 1120;
 // Bytes of shared memory one fit CTA needs: the layout, and kStaticSmem.  A
@@ -92,7 +92,8 @@ size_t fit_dynamic_smem(const DevObject &o);
 constexpr int kMaxMixedNcp = 64;
 // Facets per basis chunk of the facet sweep for a padded coefficient count.
 int chunk_facets_of(int ncp);
-// Doubles of scratch one CTA needs (derivative rows + per-curve statistics).
+// Doubles of scratch one fit in flight needs, by one CTA or a team (derivative
+// rows, per-curve statistics, partial sums, point order).
 size_t fit_scratch_doubles(const DevObject &o);
 // Padded coefficient count the kernels are compiled for.
 int padded_ncoef(int n_coef);

@@ -1,9 +1,10 @@
 // fit_kernel.cuh -- persistent FP64 Levenberg-Marquardt fit kernel for sm_100a.
 //
-// One CTA (256 threads) owns one (frequency, pole) fit at a time and runs its
-// whole LM loop on the device; CTAs pop items from a device queue, so ragged
-// iteration counts never idle the grid.  Per function evaluation (the
-// reference's mrqcof, Start.cu:535-629 + 2262-2828):
+// One CTA (256 threads) owns one (frequency, pole) fit at a time, or where
+// there are fewer fits than SMs a team of them does (a cluster of 2, 4 or 8,
+// struct Team), and runs its whole LM loop on the device; items are popped
+// from a device queue, so ragged iteration counts never idle the grid.  Per
+// function evaluation (the reference's mrqcof, Start.cu:535-629 + 2262-2828):
 //
 //   A  curv: facet areas exp(sum a_k Y_k) into shared memory  (Start.cu:421-528)
 //   B  brightness rows: a warp takes 32 points (lane = point) and sweeps every
@@ -237,7 +238,7 @@ __host__ __device__ inline int fit_mfp(int mfit)
 
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 
-// Scratch slab of one CTA, in doubles from its start:
+// Scratch slab of one fit (its CTA or team), in doubles from its start:
 //   [0, n_points * row_stride)             derivative rows
 //   [.., + n_curves * (ma + 3))            per-curve statistics
 //   [gpart, + kWarps * 36 * 64)            rank-k partial sums (16-byte aligned)
@@ -1282,10 +1283,10 @@ __device__ __forceinline__ void syrk_update(const Sh &s, int nrows, SyrkAcc &acc
     }
 }
 
-// Adds one warp's accumulators into alpha (lower triangle mirrored, stride
+// Writes one warp's accumulators into alpha (lower triangle mirrored, stride
 // ld), beta and chi^2.
-__device__ __forceinline__ void syrk_add_block(const Sh &s, int mfit, int bj, int bk, double v0, double v1,
-                                               double *dst, double *dvec, bool first)
+__device__ __forceinline__ void syrk_store_block(const Sh &s, int mfit, int bj, int bk, double v0, double v1,
+                                                 double *dst, double *dvec)
 {
     const int lane = threadIdx.x & 31, ld = s.ld;
 #pragma unroll
@@ -1294,13 +1295,12 @@ __device__ __forceinline__ void syrk_add_block(const Sh &s, int mfit, int bj, in
         const int col = 8 * bk + 2 * (lane & 3) + e;
         const double v = e ? v1 : v0;
         if (row < mfit && col <= row) {
-            const double t = first ? v : dst[row * ld + col] + v;
-            dst[row * ld + col] = t;
-            if (col != row) dst[col * ld + row] = t;
+            dst[row * ld + col] = v;
+            if (col != row) dst[col * ld + row] = v;
         } else if (row == mfit && col < mfit) {
-            dvec[col] = first ? v : dvec[col] + v;
+            dvec[col] = v;
         } else if (row == mfit && col == mfit) {
-            s.scal[S_TRIAL] = first ? v : s.scal[S_TRIAL] + v;
+            s.scal[S_TRIAL] = v;
         }
     }
 }
@@ -1360,7 +1360,7 @@ __device__ __forceinline__ void syrk_store(const Sh &s, int mfit, const SyrkAcc 
     }
 #pragma unroll
     for (int i = 0; i < kMaxBlk; ++i)
-        if (i < acc.nblk) syrk_add_block(s, mfit, acc.bj[i], acc.bk[i], acc.c[i][0], acc.c[i][1], dst, dvec, true);
+        if (i < acc.nblk) syrk_store_block(s, mfit, acc.bj[i], acc.bk[i], acc.c[i][0], acc.c[i][1], dst, dvec);
     __syncthreads();
 }
 
@@ -1786,9 +1786,10 @@ static __device__ void brightness_only(const DevObject &o, const Sh &s, double *
 // full evaluation there gives: every trial step needs it, but half of the
 // steps and more are rejected, and those need nothing else.  Measured at the
 // production object (3698 points, 512 facets, 49 coefficients):
-//   full evaluation 2.85e6 cycles, this 0.66e6; 53 % of the trial steps of
-//   its 50-iteration fits are rejected.  One wave of 50-iteration fits went
-//   from 77.9 to 57.6 ms (310 fits: 234 -> 170 ms).
+//   full evaluation 2.85e6 cycles, this 0.65e6; 52 % of the trial steps of
+//   its 50-iteration fits are rejected.  One wave of 148 such fits takes 77.7 ms
+//   with a full evaluation per trial, now 56.3 (0.5 of the gain is the
+//   solve's).
 // Leaves the facet areas (s.F), the invariants (s.inv) and the point order
 // (perm) of the trial parameters for the full evaluation that follows an
 // accepted step, the summed area in S_AREA and the summed area-weighted
@@ -2274,7 +2275,7 @@ __device__ double evaluate(const DevObject &o, const DevParams &p, const Sh &s, 
 // separate unrolled stretches without a branch, each a set of independent
 // chains: with one branch per column, values read from shared memory, a pivot
 // of 56 columns took 1630 cycles in the update of about 2250, now 1130 of 1950;
-// a solve inside a production fit 127 k -> 106 k cycles.
+// a solve inside a production fit 126 k -> 105 k cycles.
 // Returns the reference's error code: 0, 1 (pivot bookkeeping) or 2 (zero
 // pivot).  All threads must call it.  red: candidates; ctl: C_GJROW0.
 struct __align__(16) GjCand {

@@ -9,7 +9,7 @@
 // buffers) are closed to them.  ps_fit_items_noalloc runs the same persistent
 // LM fit kernel as ps_gpu_fit_items, but every device byte it touches -- the
 // object tables, the work items, the results, the queue and status words and
-// the kernel's per-CTA scratch -- lives in one file-scope __device__ array of
+// the scratch of the fits in flight -- lives in one file-scope __device__ array of
 // kNoAllocArenaBytes.  The caller passes host inputs and a host output array;
 // the call allocates nothing, on the device or on the host heap.
 //
