@@ -128,13 +128,21 @@ static KernelFn kernel_for(int ncp, int mixed)
     }
 }
 
+// Every use of a kernel allows it what the largest layout takes, not its own
+// object's: the allowance belongs to the kernel, and with the object's own size
+// a handle in another thread, of a smaller object, took it away between this and
+// the launch.
+static int allow_smem(KernelFn fn)
+{
+    return (int)cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kBlockSmem - kStaticSmem));
+}
+
 static int prepare_kernel(const DevObject &o, KernelFn *fn, size_t *smem)
 {
     *fn = kernel_for(o.ncp, o.mixed);
     if (!*fn) return (int)cudaErrorInvalidValue;
     *smem = fit_dynamic_smem(o);
-    cudaError_t e = cudaFuncSetAttribute(*fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem);
-    return (int)e;
+    return allow_smem(*fn);
 }
 
 int fit_ctas_per_sm(const DevObject &o)
@@ -164,8 +172,7 @@ int prepare_batch_kernel(const DevObject &env)
 {
     KernelFn fn = batch_kernel_for(env.ncp);
     if (!fn || env.mixed) return (int)cudaErrorInvalidValue;
-    const size_t smem = fit_dynamic_smem(env);
-    return (int)cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return allow_smem(fn);
 }
 
 int fit_batch_ctas_per_sm(const DevObject &env)
@@ -211,7 +218,7 @@ struct TeamLaunch {
         cfg.stream = (cudaStream_t)stream;
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
-        return (int)cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        return allow_smem(fn);
     }
 };
 

@@ -82,6 +82,7 @@ enum StatusBits : int {
 // kernel has none, the teams' kernel about 700 bytes (TeamShared), the batch kernel
 // the item's object and constants.
 constexpr size_t kStaticSmem = 1120;
+constexpr size_t kBlockSmem = 232448;  // shared memory one block may have (sm_100)
 // Bytes of shared memory one fit CTA needs: the layout, and kStaticSmem.  A
 // layout is chosen by this, so that each kernel can run it; the launches ask
 // for the layout alone (fit_dynamic_smem).
@@ -132,7 +133,7 @@ int launch_fit_teams(const DevObject &o, const DevParams &p, const FitItem *item
 // layout: n_fac, mfit, n_curves, row_stride) and the common tile_rows and
 // cstat_smem; d_objs / d_prms are the objects' tables and constants on the
 // device, and an item's pole field is pole | object << 8.
-// prepare_batch_kernel sets the kernel's shared-memory limit (once, before
+// prepare_batch_kernel sets the shared memory the kernel is allowed (before
 // launching or capturing); launch_fits_batch only enqueues the launch.
 int prepare_batch_kernel(const DevObject &env);
 int fit_batch_ctas_per_sm(const DevObject &env);
